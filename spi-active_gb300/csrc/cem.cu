@@ -15,6 +15,7 @@ int cem_sample_impl(spi_engine* e) {
   int rc = refresh_after_realloc(e);
   if (rc) return rc;
   e->N = e->cem_n;
+  e->population = true;
   CemState* st = (CemState*)e->cem.p;
   cem_sample_kernel<<<dim3(blocks_for(e->N, 128), 1), 128, 0, e->stream>>>(st);
   cudaError_t ce = cudaGetLastError();
@@ -108,6 +109,7 @@ int spi_cem_init(spi_engine* e, const spi_cem_config* c) {
   if (ce != cudaSuccess) return cuda_error(ce, "spi_cem_init: upload");
   e->N = c->n_samples;
   e->cem_n = c->n_samples;
+  e->population = true;
   e->cem_ready = true;
   if (e->graph_exec) { cudaGraphExecDestroy(e->graph_exec); e->graph_exec = nullptr; }
   e->seen_generation = e->theta.generation + e->cost.generation + e->partial.generation + e->comp.generation +

@@ -455,6 +455,25 @@ template <int AX, int RM, class T> SPI_INL void ri_to_parent_art_acc(const RI<T>
 struct alignas(16) F4 { float x, y, z, w; };
 constexpr int kLegSlots = 14;
 
+// A leg's constants as leg_condense (leg_hip.cuh) reads them, four to a 16-byte slot; 13 slots, so that the four legs' copies of a slot
+// start in different shared-memory banks.
+template <class S> struct alignas(16) HipLeg {
+  S x0, y0, y1, z2;            // hip origin (x0, y0, 0), thigh origin (0, y1, 0), calf origin (0, 0, z2)
+  S kd[3], m0;                 // joint damping; hip mass
+  S iv[3], m12;                // 1 / velocity limit (0: no limit); thigh + calf mass
+  S h0x, h0y, h0z, m2;         // hip first moment; calf mass
+  S J0xx, J0yy, J0zz, J0xy;    // hip second moments about o0
+  S J0xz, J0yz, h1x, h1z;      // thigh about o0, thigh axes: first moment,
+  S h1y, P1, D1, X1;           //   (Jxx + Jzz) / 2, (Jxx - Jzz) / 2, Jxz,
+  S J1xy, J1yz, yy12, h2x;     //   Jxy, Jyz; Jyy of thigh (about o0) + calf (about its joint)
+  S h2y, h2z, P2, D2;          // calf about its joint, calf axes: as the thigh
+  S X2, J2xy, J2yz, hf2;       //   hf2 = (foot z)^2 / 2
+  S c0x, c0y, c0z, c1x;        // the leg's two base-box corners
+  S c1y, c1z, pad[2];
+  S pad2[4];
+};
+static_assert(sizeof(HipLeg<float>) == 13 * 16, "HipLeg: 13 slots");
+
 struct DevModel {
   // The per-leg constants phase A reads, leg-major, four to a 16-byte slot, so that one leg's
   // are contiguous (one 128-bit load per slot) and the four legs' copies of a slot sit 56
@@ -464,6 +483,7 @@ struct DevModel {
   //          (1 / vlim is 0 without the torque-speed limit)
   //   12, 13 the leg's two base-box corners: (c0 x, c0 y, c0 z, c1 x), (c1 y, c1 z, 0, 0)
   F4 legc[4][kLegSlots];
+  HipLeg<float> hip[4];
   // per leg body k (0 hip, 1 thigh, 2 calf), component, leg: [k][c][leg] (the same constants
   // as the source arrays of legc, for the host-side formulations)
   float org[3][3][4];
@@ -974,9 +994,10 @@ template <class T> SPI_INL LegOut<T> base_terms(const BaseParams<T>& bp, const B
 }
 
 // Base solve and base integration from the total articulated inertia IA and bias force pA at
-// the base. Returns the base acceleration with gravity removed.
+// the base, all but the position: d receives the base's displacement. Returns the base
+// acceleration with gravity removed.
 template <class T>
-SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B) {
+SPI_INL SV<T> base_solve_step(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B, V3<T>& d) {
   // 6x6 symmetric matrix in (w; v) order, Cholesky L L^T, solve IA a = -pA
   T Mx[6][6];
   Mx[0][0] = IA.A.xx; Mx[1][1] = IA.A.yy; Mx[2][2] = IA.A.zz;
@@ -991,10 +1012,10 @@ SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, B
   T invL[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    T d = Mx[j][j];
+    T piv = Mx[j][j];
 #pragma unroll
-    for (int k = 0; k < j; ++k) d = d - Mx[j][k] * Mx[j][k];
-    T inv = T(1) / m_sqrt(d);
+    for (int k = 0; k < j; ++k) piv = piv - Mx[j][k] * Mx[j][k];
+    T inv = T(1) / m_sqrt(piv);
     invL[j] = inv;
 #pragma unroll
     for (int i = j + 1; i < 6; ++i) {
@@ -1034,7 +1055,14 @@ SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, B
   T inv = T(1) / m_sqrt(nx * nx + ny * ny + nz * nz + nw * nw);
   B.qx = nx * inv; B.qy = ny * inv; B.qz = nz * inv; B.qw = nw * inv;
   B.R = quat_to_R(B.qx, B.qy, B.qz, B.qw);
-  B.p = B.p + dt * mul(B.R, B.nu.v);
+  d = dt * mul(B.R, B.nu.v);
+  return a0;
+}
+template <class T>
+SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B) {
+  V3<T> d;
+  const SV<T> a0 = base_solve_step(M, IA, pA, B, d);
+  B.p = B.p + d;
   return a0;
 }
 
@@ -1042,9 +1070,7 @@ SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, B
 // Phase C: joint accelerations of one leg from the base acceleration, then joint integration:
 // qdd = L^-T (y - K'^T a0).
 // ---------------------------------------------------------------------------
-template <class T, class WK>
-SPI_INL void phase_c(const DevModel& M, int leg, const SV<T>& a0, const WK& W, LegState<T>& L) {
-  (void)leg;
+template <class T, class WK> SPI_INL void joint_accel(const SV<T>& a0, const WK& W, T qdd[3]) {
   T w[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -1054,10 +1080,15 @@ SPI_INL void phase_c(const DevModel& M, int leg, const SV<T>& a0, const WK& W, L
     w[k] = vx - q.w.x * a0.w.x - q.w.y * a0.w.y - q.w.z * a0.w.z - q.v.y * a0.v.y - q.v.z * a0.v.z;
   }
   const T w0 = w[0], w1 = w[1], w2 = w[2];
-  T qdd[3];
   qdd[2] = w2;
   qdd[1] = w1 - W.l21 * qdd[2];
   qdd[0] = w0 - W.l10 * qdd[1] - W.l20 * qdd[2];
+}
+template <class T, class WK>
+SPI_INL void phase_c(const DevModel& M, int leg, const SV<T>& a0, const WK& W, LegState<T>& L) {
+  (void)leg;
+  T qdd[3];
+  joint_accel(a0, W, qdd);
   T dt = T(M.dt);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {

@@ -7,6 +7,7 @@
 
 #include "common.h"
 #include "engine_impl.h"
+#include "eval.h"
 #include "items.h"
 #include "model.h"
 #include "rollout.cuh"
@@ -68,7 +69,14 @@ int spi::run_impl(spi_engine* e, float* trace) {
   const long long warps = (long long)e->N * G;
   const unsigned grid = blocks_for(warps, 4);
   unsigned long long* bad = (unsigned long long*)e->bad.p;
-  if (!trace && (e->layout == SPI_LAYOUT_LANE || e->layout == SPI_LAYOUT_QUAD)) {
+  if (trace) {
+    rollout_kernel<true, 3><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
+                                                         e->partial.f(), trace, bad);
+  } else if (e->layout == SPI_LAYOUT_LANE && !e->population) {
+    const EvalArgs a{win, e->theta.f(), e->partial.f(), e->N, G, bad};
+    const cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);
+    if (ce != cudaSuccess) return cuda_error(ce, "rollout launch");
+  } else if (e->layout != SPI_LAYOUT_BLOCK) {
     // the server's rollout kernel on a table of one slot (items.h), one warp per work item
     SlotDesc d{};
     d.win = win;
@@ -89,7 +97,7 @@ int spi::run_impl(spi_engine* e, float* trace) {
       ce = items_launch(e->layout, e->min_blocks, e->host_model, e->d_model, single_tables(tab), 0, (int)ctas, bad,
                         e->stream);
     if (ce != cudaSuccess) return cuda_error(ce, "rollout launch");
-  } else if (!trace && e->layout == SPI_LAYOUT_BLOCK) {
+  } else {
     if (e->min_blocks == 4)
       rollout_block_kernel<4><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
                                                             e->partial.f(), bad);
@@ -99,9 +107,6 @@ int spi::run_impl(spi_engine* e, float* trace) {
     else
       rollout_block_kernel<3><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
                                                             e->partial.f(), bad);
-  } else {
-    rollout_kernel<true, 3><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
-                                                         e->partial.f(), trace, bad);
   }
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return cuda_error(ce, "rollout_kernel launch");
@@ -137,6 +142,10 @@ int spi_create(const spi_robot* robot, spi_engine** out) {
   if (!rc) rc = e->items.reserve(sizeof(SingleTable));
   if (rc) { cudaFree(e->d_model); delete e; return rc; }
   cudaMemset(e->bad.p, 0, sizeof(unsigned long long));
+  int dev = 0;
+  ce = cudaGetDevice(&dev);
+  if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev);
+  if (ce != cudaSuccess) { spi_destroy(e); return cuda_error(ce, "spi_create: device"); }
   // default kernel: the lane layout at the 168-register cap (the fastest on the C1 workload)
   if ((rc = spi_set_kernel_layout(e, SPI_LAYOUT_LANE)) || (rc = spi_set_kernel_config(e, 3))) {
     spi_destroy(e);
@@ -201,6 +210,7 @@ int spi_set_theta(spi_engine* e, const float* theta, int N) {
                                    cudaMemcpyDeviceToDevice, e->stream);
   if (ce != cudaSuccess) return cuda_error(ce, "spi_set_theta");
   e->N = N;
+  e->population = false;
   e->ran = false;
   return SPI_OK;
 }
@@ -221,7 +231,8 @@ int spi_set_kernel_layout(spi_engine* e, int layout) {
     return set_error(SPI_EINVAL, "spi_set_kernel_layout: layout %d not 0/1/2", layout);
   if (layout == SPI_LAYOUT_LANE) {
     // the parking area is above the 48 KB default for dynamic shared memory
-    const cudaError_t ce = items_prepare_lane();
+    cudaError_t ce = items_prepare_lane();
+    if (ce == cudaSuccess) ce = eval_prepare();
     if (ce != cudaSuccess) return cuda_error(ce, "spi_set_kernel_layout: shared-memory attribute");
   } else if (e->min_blocks < 3) {
     e->min_blocks = 3;

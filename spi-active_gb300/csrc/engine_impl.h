@@ -10,12 +10,14 @@
 struct spi_engine {
   spi::DevModel host_model;
   spi::DevModel* d_model = nullptr;
+  int sms = 0;                             // SMs of the engine's device
   cudaStream_t stream = nullptr;
   spi::DeviceBuf init, act, tgt, weight;   // windows, structure-of-arrays
   int W = 0, H = 0;
   float norm = 1.f;
   spi::DeviceBuf theta;                    // [N][13]
   int N = 0;
+  bool population = false;                 // the batch is the CEM's population (spi_run keeps its kernels)
   spi::DeviceBuf partial, comp, cost;      // [N][G][9], [N][9], [N]
   spi::DeviceBuf bad;                      // one unsigned long long
   int cost_mode = 1;

@@ -121,6 +121,22 @@ static void substep(const DevModel& M, BaseState<T>& B, LegState<T> L[4], const 
   }
 }
 
+// One substep by the legs condensed in the hip frame (leg_hip.cuh), act = the joint targets.
+template <class T, class S>
+static void substep_hip(const DevModel& M, const HipLeg<S> hip[4], BaseState<T>& B, LegState<T> L[4],
+                        const BaseParams<T>& bp, const LegParams<T> lp[4], const T act[12]) {
+  LegWork<T> W[4];
+  LegOut<T> sum = base_terms(bp, B);
+  const bool corners = corners_may_touch(M, B);
+  for (int leg = 0; leg < 4; ++leg) {
+    LegOut<T> o;
+    leg_condense<kMotorRuntime>(M, hip[leg], B, L[leg], leg_gains(M, lp[leg], leg), act + 3 * leg, W[leg], o, corners);
+    add_out(sum, o);
+  }
+  const SV<T> a0 = base_solve(M, sum.I, sum.p, B);
+  for (int leg = 0; leg < 4; ++leg) phase_c(M, leg, a0, W[leg], L[leg]);
+}
+
 template <class T>
 static void load_rollout(const DevModel& M, const double* x, const double* th, BaseState<T>& B,
                          LegState<T> L[4], BaseParams<T>& bp, LegParams<T> lp[4]) {
@@ -339,13 +355,19 @@ static int hostemu_residual(const spi_robot* robot, const double* state, const d
   return SPI_OK;
 }
 
-template <bool ABA, class T>
+// Which form of the leg equations a host rollout runs: the condensed legs of dynamics.cuh, the
+// articulated-body algorithm of the oracle, or the hip-frame legs of leg_hip.cuh.
+constexpr int kCondensed = 0, kAba = 1, kHip = 2;
+template <int FORM, class T>
 static int hostemu_rollout(const spi_robot* robot, const double* init, const double* actions,
                            const double* theta, int nb, int H, double* trace) {
   DevModel M;
   const char* why = "";
   int rc = build_dev_model(*robot, &M, &why);
   if (rc) return rc;
+  HipLeg<T> hip[4];
+  if (FORM == kHip)
+    for (int leg = 0; leg < 4; ++leg) hip[leg] = hip_leg_constants<T>(*robot, leg);
   for (int b = 0; b < nb; ++b) {
     BaseState<T> B;
     LegState<T> L[4];
@@ -355,8 +377,11 @@ static int hostemu_rollout(const spi_robot* robot, const double* init, const dou
     for (int h = 0; h < H; ++h) {
       const double* a = actions + ((size_t)b * H + h) * 12;
       T act[12];
-      for (int j = 0; j < 12; ++j) act[j] = ABA ? T(a[j]) : joint_target(M, j % 3, j / 3, T(a[j]));
-      for (int s = 0; s < M.decimation; ++s) substep<ABA>(M, B, L, bp, lp, act);
+      for (int j = 0; j < 12; ++j) act[j] = FORM == kAba ? T(a[j]) : joint_target(M, j % 3, j / 3, T(a[j]));
+      for (int s = 0; s < M.decimation; ++s) {
+        if (FORM == kHip) substep_hip(M, hip, B, L, bp, lp, act);
+        else substep<FORM == kAba>(M, B, L, bp, lp, act);
+      }
       double* out = trace + ((size_t)b * H + h) * SPI_STATE_DIM;
       T s13[13];
       base_to_world(B, s13);
@@ -400,16 +425,22 @@ extern "C" {
 // theta [B][13] -> trace [B][H][37]; FP64, and FP32 (the device's arithmetic type).
 int spi_hostemu_rollout(const spi_robot* robot, const double* init, const double* actions,
                         const double* theta, int nb, int H, double* trace) {
-  return hostemu_rollout<false, double>(robot, init, actions, theta, nb, H, trace);
+  return hostemu_rollout<kCondensed, double>(robot, init, actions, theta, nb, H, trace);
 }
 int spi_hostemu_rollout_f32(const spi_robot* robot, const double* init, const double* actions,
                             const double* theta, int nb, int H, double* trace) {
-  return hostemu_rollout<false, float>(robot, init, actions, theta, nb, H, trace);
+  return hostemu_rollout<kCondensed, float>(robot, init, actions, theta, nb, H, trace);
 }
 // The same rollouts with the legs by the articulated-body algorithm (FP64).
 int spi_hostemu_rollout_aba(const spi_robot* robot, const double* init, const double* actions,
                             const double* theta, int nb, int H, double* trace) {
-  return hostemu_rollout<true, double>(robot, init, actions, theta, nb, H, trace);
+  return hostemu_rollout<kAba, double>(robot, init, actions, theta, nb, H, trace);
+}
+
+// The same rollouts with the legs condensed in the hip frame (FP64), the rollout kernels' form.
+int spi_hostemu_rollout_hip(const spi_robot* robot, const double* init, const double* actions,
+                            const double* theta, int nb, int H, double* trace) {
+  return hostemu_rollout<kHip, double>(robot, init, actions, theta, nb, H, trace);
 }
 
 // FP operations the kernel executes in one physics substep (whole rollout, phase B counted

@@ -5,7 +5,7 @@
 #include <math.h>
 #include <string.h>
 
-#include "dynamics.cuh"
+#include "leg_hip.cuh"
 
 namespace spi {
 
@@ -88,6 +88,7 @@ inline int build_dev_model(const spi_robot& r, DevModel* M, const char** why) {
     *why = "sim_dt must be > 0 and decimation in [1, 64]"; return SPI_EINVAL;
   }
   if (!(r.friction_vel > 0.0f)) { *why = "friction_vel must be > 0"; return SPI_EINVAL; }
+  for (int leg = 0; leg < 4; ++leg) M->hip[leg] = hip_leg_constants<float>(r, leg);
   M->fric_k2 = (float)(2.0 / (log(2.0) * (double)r.friction_vel));
   if (r.inertia_follows_mass && !(r.base_mass_nominal > 0.0f)) {
     *why = "base_mass_nominal must be > 0 with inertia_follows_mass"; return SPI_EINVAL;

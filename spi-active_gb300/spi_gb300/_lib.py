@@ -98,6 +98,8 @@ def hostemu_lib():
         lib.spi_hostemu_rollout_f32.argtypes = lib.spi_hostemu_rollout.argtypes
         lib.spi_hostemu_rollout_aba.restype = c_int
         lib.spi_hostemu_rollout_aba.argtypes = lib.spi_hostemu_rollout.argtypes
+        lib.spi_hostemu_rollout_hip.restype = c_int
+        lib.spi_hostemu_rollout_hip.argtypes = lib.spi_hostemu_rollout.argtypes
         lib.spi_hostemu_count_ops.restype = c_int
         lib.spi_hostemu_count_ops.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p,
                                               POINTER(ctypes.c_longlong), POINTER(ctypes.c_longlong)]

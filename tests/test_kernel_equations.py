@@ -122,6 +122,27 @@ def test_condensed_legs_equal_articulated_body_algorithm(built):
     assert np.abs(emu - out).max() < 1e-9
 
 
+@pytest.mark.parametrize("kw", [dict(), dict(torque_speed=False), dict(tanh_a=(15.0, 18.0, 25.0), hip_action_scale=0.5),
+                                dict(base_contact=False, motor_gain=(0.9, 1.1, 1.05))])
+def test_hip_frame_legs_equal_articulated_body_algorithm(built, kw):
+    """The legs condensed in the hip frame (csrc/leg_hip.cuh) and the oracle's articulated-body
+    algorithm, both in FP64 with the same constants, agree to rounding: feet in and out of contact,
+    base-box corners on the ground, each motor model."""
+    from spi_gb300 import _lib, robot
+    _, x0, acts, th = _inputs(16, B=24, H=12)
+    x0[:8, 2] = 0.26
+    x0[8:12, 2] = 0.08
+    r = robot.to_struct(robot.SimConfig(**kw))
+    x0c, ac, tc = (np.ascontiguousarray(a, dtype=np.float64) for a in (x0, acts, th))
+    out = []
+    for form in ("aba", "hip"):
+        o = np.zeros((24, 12, 37))
+        fn = getattr(_lib.hostemu_lib(), f"spi_hostemu_rollout_{form}")
+        assert fn(ctypes.byref(r), x0c.ctypes.data, ac.ctypes.data, tc.ctypes.data, 24, 12, o.ctypes.data) == 0
+        out.append(o)
+    assert np.abs(out[0] - out[1]).max() < 1e-9
+
+
 def test_kernel_vs_oracle_with_urdf_constants(built):
     """Float32 model constants move states by < 1e-5 (well inside the 1e-4 parity bar)."""
     cfg, x0, acts, th = _inputs(13)
