@@ -121,106 +121,164 @@ __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __rest
   }
 }
 
-// F[n] = sum_w J^T diag(q) J (K x K, FP32 accumulation); one CTA per sample.
-__global__ void fisher_kernel(const float* __restrict__ J, int N, int W, int K, const float* __restrict__ q,
-                              float* __restrict__ F) {
-  const int n = blockIdx.x;
-  const int nent = K * K;
-  for (int e = threadIdx.x; e < nent; e += blockDim.x) {
-    const int p = e / K, r = e % K;
-    if (r < p) continue;
-    float acc = 0.f;
-    for (int w = 0; w < W; ++w) {
-      const float* Jw = J + (((size_t)n * W + w) * SPI_STATE_DIM) * K;
-#pragma unroll 1
-      for (int i = 0; i < SPI_STATE_DIM; ++i) acc += (q ? q[i] : 1.f) * Jw[i * K + p] * Jw[i * K + r];
-    }
-    F[(size_t)n * nent + p * K + r] = acc;
-    F[(size_t)n * nent + r * K + p] = acc;
-  }
-}
+// ---------------------------------------------------------------------------
+// Fisher information: F[n] = sum_w J^T diag(q) J, log det(F + eps I) and trace(F), two samples a CTA.
+//
+// J is read once, coalesced, kFisherRows rows at a time (the next rows are on their way in registers while
+// these are summed), into shared memory in the layout the accumulation reads; the sums run from there
+// in row order, as one chain per entry (FP32) or per 8-column tile of the m16n8k16 product (tensor
+// cores), so the staging does not show in a result. The scores follow in the same launch, both
+// samples on one warp: an FP64 instruction holds GB300's FP64 pipe for sixteen cycles whatever its
+// lanes do, and a sample has 13 rows. 512 samples x 8 windows x 13 parameters, BF16: 115 -> 16.5 us.
+// ---------------------------------------------------------------------------
+constexpr int kFisherRows = 128;                 // rows of J staged at a time (a multiple of 16)
+constexpr int kFisherPitch = kFisherRows / 2 + 4;   // words per parameter of the BF16 tile; 4 mod 32: conflict-free
+constexpr int kFisherThreads = 128;              // per sample
+constexpr int kFisherPer = kFisherRows * SPI_THETA_DIM / kFisherThreads;   // elements a thread stages
 
-// F[n] = sum_w J^T diag(q) J on tensor cores: one warp per sample, BF16 operands, FP32
-// accumulation, mma.sync m16n8k16 (A = (Q^1/2 J)^T as a 16 x 16 row-major tile, B = Q^1/2 J as a
-// 16 x 8 column-major tile, two n-tiles cover the 16 padded parameters). Rows of J are consumed
-// 16 at a time; rows past W * 37 and parameters past K are zero.
-__device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<unsigned*>(&v);
-}
-__device__ __forceinline__ float jq(const float* __restrict__ Jn, const float* __restrict__ q, int rows, int K,
-                                    int r, int p) {
-  if (r >= rows || p >= K) return 0.f;
-  const float w = q ? sqrtf(q[r % SPI_STATE_DIM]) : 1.f;
-  return w * Jn[(size_t)r * K + p];
-}
-__global__ void fisher_mma_kernel(const float* __restrict__ J, int N, int W, int K, const float* __restrict__ q,
-                                  float* __restrict__ F) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= N) return;                        // uniform per warp
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const float* Jn = J + (size_t)warp * W * SPI_STATE_DIM * K;
-  const int rows = W * SPI_STATE_DIM;
-  float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < rows; k0 += 16) {
-    // A[m][k] = Jq[k0 + k][m]: rows m = g, g + 8; cols k = 2t, 2t + 1, 2t + 8, 2t + 9
-    const unsigned a0 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t, g), jq(Jn, q, rows, K, k0 + 2 * t + 1, g));
-    const unsigned a1 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t, g + 8), jq(Jn, q, rows, K, k0 + 2 * t + 1, g + 8));
-    const unsigned a2 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t + 8, g), jq(Jn, q, rows, K, k0 + 2 * t + 9, g));
-    const unsigned a3 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t + 8, g + 8),
-                                  jq(Jn, q, rows, K, k0 + 2 * t + 9, g + 8));
+// log det(F + eps I) by an FP64 L D L^T and trace(F), row i on lane i of a half-warp. A column's pivot and
+// entries go round by shuffles; each entry's subtractions run in the order k = 0 .. j - 1. logdet / trace
+// null: not written.
+__device__ __forceinline__ void fisher_scores(const float* F, int K, double eps, double* logdet, double* trace) {
+  const int i = threadIdx.x & 15;
+  double row[SPI_THETA_DIM];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      // B[k][n] = Jq[k0 + k][8 nt + n]: k = 2t, 2t + 1 (b0) and 2t + 8, 2t + 9 (b1); n = g
-      const int n = 8 * nt + g;
-      const unsigned b0 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t, n), jq(Jn, q, rows, K, k0 + 2 * t + 1, n));
-      const unsigned b1 = pack_bf16(jq(Jn, q, rows, K, k0 + 2 * t + 8, n), jq(Jn, q, rows, K, k0 + 2 * t + 9, n));
-      float* c = nt ? c1 : c0;
-      asm volatile(
-          "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-          "{%0, %1, %2, %3};\n"
-          : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-          : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-  }
-  // D fragment: rows g and g + 8, cols 2t and 2t + 1 of each n-tile
-  float* Fn = F + (size_t)warp * K * K;
-#pragma unroll
-  for (int nt = 0; nt < 2; ++nt) {
-    const float* c = nt ? c1 : c0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int m = g + (e >= 2 ? 8 : 0), n = 8 * nt + 2 * t + (e & 1);
-      if (m < K && n < K) Fn[m * K + n] = c[e];
-    }
-  }
-}
-
-// log det(F + eps I) by FP64 Cholesky, and trace(F); one thread per sample.
-__global__ void logdet_kernel(const float* __restrict__ F, int N, int K, double eps, double* __restrict__ logdet,
-                              double* __restrict__ trace) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  double L[SPI_THETA_DIM * SPI_THETA_DIM];
-  const float* f = F + (size_t)n * K * K;
-  double ld = 0.0, tr = 0.0;
+  for (int j = 0; j < SPI_THETA_DIM; ++j)
+    row[j] = i < K && j < K ? (double)F[i * K + j] + (j == i ? eps : 0.0) : 0.0;
+  const double diag = i < K ? (double)F[i * K + i] : 0.0;
+  double pivot = 1.0, tr = 0.0;
   bool ok = true;
-  for (int j = 0; j < K; ++j) {
-    double d = (double)f[j * K + j] + eps;
-    tr += (double)f[j * K + j];
-    for (int k = 0; k < j; ++k) d -= L[j * K + k] * L[j * K + k];
-    if (!(d > 0.0)) { ok = false; break; }
-    const double ljj = sqrt(d);
-    L[j * K + j] = ljj;
-    ld += 2.0 * log(ljj);
-    for (int i = j + 1; i < K; ++i) {
-      double s = (double)f[i * K + j];
-      for (int k = 0; k < j; ++k) s -= L[i * K + k] * L[j * K + k];
-      L[i * K + j] = s / ljj;
+#pragma unroll
+  for (int j = 0; j < SPI_THETA_DIM; ++j) {
+    if (j < K) {                                  // uniform
+      const double t = __shfl_sync(0xffffffffu, diag, j, 16);
+      if (ok) tr += t;
+      const double d = __shfl_sync(0xffffffffu, row[j], j, 16);
+      ok = ok && d > 0.0;
+      if (i == j) pivot = d;
+      const double l = row[j] * (1.0 / d);
+#pragma unroll
+      for (int k = j + 1; k < SPI_THETA_DIM; ++k)
+        if (k < K) row[k] -= l * __shfl_sync(0xffffffffu, row[j], k, 16);
     }
   }
-  if (logdet) logdet[n] = ok ? ld : -INFINITY;
-  if (trace) trace[n] = tr;
+  const double lg = log(pivot);
+  double ld = 0.0;
+  for (int j = 0; j < K; ++j) ld += __shfl_sync(0xffffffffu, lg, j, 16);
+  if (i == 0) {
+    if (logdet) *logdet = ok ? ld : -INFINITY;
+    if (trace) *trace = tr;
+  }
+}
+
+// TC = false: FP32 on the CUDA cores, one entry (p, r >= p) a thread: acc += (q J_p) J_r over the rows.
+// TC = true: BF16 operands (Q^1/2 J), FP32 accumulation, mma.sync m16n8k16 by one warp: A = (Q^1/2 J)^T
+// as a 16 x 16 tile, B = Q^1/2 J as two 16 x 8 tiles (the same registers: A's row groups are B's columns).
+// Rows past W * 37 and parameters past K are zero. (13 parameters fill a fifth of the smallest tcgen05
+// tile, M = 64; the product is a few microseconds of one warp here.)
+template <bool TC>
+__global__ void __launch_bounds__(2 * kFisherThreads) fisher_kernel(const float* __restrict__ J, int N, int W, int K,
+                                                                    const float* __restrict__ q, double eps,
+                                                                    float* __restrict__ F, double* __restrict__ logdet,
+                                                                    double* __restrict__ trace) {
+  constexpr int kWords = TC ? 16 * kFisherPitch : 2 * kFisherRows * SPI_THETA_DIM;
+  __shared__ __align__(16) unsigned tiles[2][kWords];
+  __shared__ float s_q[SPI_STATE_DIM];
+  __shared__ float s_F[2][SPI_THETA_DIM * SPI_THETA_DIM];
+  const int half = threadIdx.x / kFisherThreads, tid = threadIdx.x % kFisherThreads;
+  const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const bool live = (int)(2 * blockIdx.x + half) < N;
+  const int n = live ? 2 * blockIdx.x + half : N - 1;          // the odd sample out runs a copy of the last
+  unsigned* tile = tiles[half];
+  const int rows = W * SPI_STATE_DIM;
+  const float* Jn = J + (size_t)n * rows * K;
+  if (threadIdx.x < SPI_STATE_DIM) s_q[tid] = q ? (TC ? sqrtf(q[tid]) : q[tid]) : 1.f;
+  if (TC)
+    for (int i = tid; i < kWords; i += kFisherThreads) tile[i] = 0u;
+  // this thread's entry of the FP32 sums
+  const int nent = K * (K + 1) / 2;
+  int ep = 0, er = tid;
+  while (ep < K && er >= K - ep) { er -= K - ep; ++ep; }
+  er += ep;
+  const unsigned inv_K = 65536u / K + 1;                       // i / K for i < kFisherRows * 13
+  float acc = 0.f, c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+  float next[kFisherPer];
+#pragma unroll
+  for (int e = 0; e < kFisherPer; ++e) {
+    const int i = e * kFisherThreads + tid;
+    next[e] = i < min(kFisherRows, rows) * K ? __ldg(Jn + i) : 0.f;
+  }
+  for (int r0 = 0; r0 < rows; r0 += kFisherRows) {
+    const int m = min(kFisherRows, rows - r0), ahead = min(kFisherRows, rows - r0 - kFisherRows) * K;
+    __syncthreads();                              // the tile is free (and, at first, s_q and the zeros are set)
+#pragma unroll
+    for (int e = 0; e < kFisherPer; ++e) {
+      const int i = e * kFisherThreads + tid;
+      if (i < m * K) {
+        const int r = (int)((unsigned)i * inv_K >> 16), p = i - r * K;
+        const float v = next[e], w = s_q[(r0 + r) % SPI_STATE_DIM];
+        if (TC) {
+          reinterpret_cast<__nv_bfloat16*>(tile)[p * 2 * kFisherPitch + r] = __float2bfloat16_rn(w * v);
+        } else {
+          reinterpret_cast<float*>(tile)[i] = w * v;
+          reinterpret_cast<float*>(tile)[kFisherRows * SPI_THETA_DIM + i] = v;
+        }
+      }
+      next[e] = i < ahead ? __ldg(Jn + (size_t)(r0 + kFisherRows) * K + i) : 0.f;
+    }
+    if (TC && m < kFisherRows)                    // the rows up to the next multiple of 16 are zero
+      for (int i = tid; i < 16 * 16; i += kFisherThreads) {
+        const int p = i >> 4, r = m + (i & 15);
+        if (r < ((m + 15) & ~15)) reinterpret_cast<__nv_bfloat16*>(tile)[p * 2 * kFisherPitch + r] = __float2bfloat16_rn(0.f);
+      }
+    __syncthreads();
+    if (TC) {
+      if (tid < 32)
+        for (int k0 = 0; k0 < m; k0 += 16) {
+          // (rows k0 + 2t, 2t + 1) and (k0 + 2t + 8, 2t + 9) of parameters g and g + 8
+          const unsigned* u = tile + g * kFisherPitch + k0 / 2 + t;
+          const unsigned* v = u + 8 * kFisherPitch;
+          const unsigned a0 = u[0], a1 = v[0], a2 = u[4], a3 = v[4];
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            float* c = nt ? c1 : c0;
+            const unsigned b0 = nt ? a1 : a0, b1 = nt ? a3 : a2;
+            asm volatile(
+                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                "{%0, %1, %2, %3};\n"
+                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+          }
+        }
+    } else if (tid < nent) {
+      const float* x = reinterpret_cast<const float*>(tile) + ep;
+      const float* y = reinterpret_cast<const float*>(tile) + kFisherRows * SPI_THETA_DIM + er;
+#pragma unroll 16
+      for (int r = 0; r < m; ++r) acc = fmaf(x[r * K], y[r * K], acc);
+    }
+  }
+  float* Fs = s_F[half];
+  if (TC) {
+    // D fragment: rows g and g + 8, cols 2t and 2t + 1 of each n-tile
+    if (tid < 32)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = g + (e >= 2 ? 8 : 0), j = 8 * nt + 2 * t + (e & 1);
+          if (i < K && j < K) Fs[i * K + j] = (nt ? c1 : c0)[e];
+        }
+  } else if (tid < nent) {
+    Fs[ep * K + er] = acc;
+    Fs[er * K + ep] = acc;
+  }
+  __syncthreads();
+  if (live)
+    for (int i = tid; i < K * K; i += kFisherThreads) F[(size_t)n * K * K + i] = Fs[i];
+  if (threadIdx.x < 32 && (logdet || trace)) {
+    const int h = threadIdx.x >> 4, s = 2 * blockIdx.x + h;
+    fisher_scores(s_F[h], K, eps, logdet && s < N ? logdet + s : nullptr, trace && s < N ? trace + s : nullptr);
+  }
 }
 
 }  // namespace
@@ -258,10 +316,9 @@ int spi_fisher_ex(const float* J, int N, int W, int K, const float* state_weight
     return set_error(SPI_EINVAL, "spi_fisher: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   if (tensor_cores)
-    fisher_mma_kernel<<<(N + 3) / 4, 128, 0, s>>>(J, N, W, K, state_weight, F);
+    fisher_kernel<true><<<(N + 1) / 2, 2 * kFisherThreads, 0, s>>>(J, N, W, K, state_weight, eps, F, logdet, trace);
   else
-    fisher_kernel<<<N, 128, 0, s>>>(J, N, W, K, state_weight, F);
-  if (logdet || trace) logdet_kernel<<<(N + 127) / 128, 128, 0, s>>>(F, N, K, eps, logdet, trace);
+    fisher_kernel<false><<<(N + 1) / 2, 2 * kFisherThreads, 0, s>>>(J, N, W, K, state_weight, eps, F, logdet, trace);
   cudaError_t ce = cudaGetLastError();
   return ce == cudaSuccess ? SPI_OK : cuda_error(ce, "spi_fisher");
 }
