@@ -232,8 +232,17 @@ template <class T> struct LegTape {
   V3<T> vf, Fc;                      // foot velocity and contact force (calf frame)
 };
 
+// The pose's part of the tape: joint sines and cosines, and the world vertical down the leg.
+template <class T> SPI_INL void leg_pose(const BaseState<T>& B, const LegState<T>& L, LegTape<T>& t) {
+  for (int k = 0; k < 3; ++k) m_sincos(L.q[k], &t.s[k], &t.c[k]);
+  t.g0 = row(B.R, 2);
+  t.g1 = rotT<0>(t.c[0], t.s[0], t.g0);
+  t.g2 = rotT<1>(t.c[1], t.s[1], t.g1);
+  t.g3 = rotT<1>(t.c[2], t.s[2], t.g2);
+}
+
 // r[k]: joint k's residual f_k . S_k + arm qdd_k - tau_k; fb: the leg's force on the base
-// (X_0^T f_0). tgt: the three joint targets (joint_target of the actions).
+// (X_0^T f_0). tgt: the three joint targets (joint_target of the actions). t holds leg_pose.
 template <int MS, class T>
 SPI_INL void leg_residual(const DevModel& M, int leg, const BaseState<T>& B, const LegState<T>& L,
                           const LegParams<T>& P, const T tgt[3], const SV<T>& a0, const T qdd[3], LegTape<T>& t,
@@ -242,19 +251,12 @@ SPI_INL void leg_residual(const DevModel& M, int leg, const BaseState<T>& B, con
   const V3<T> r0 = lc_org<T>(lc, 0), r1 = lc_org<T>(lc, 1), r2 = lc_org<T>(lc, 2);
   const V3<T> rf = v3(T(0), T(0), T(M.foot[2]));
   T tau[3];
-  for (int k = 0; k < 3; ++k) {
-    tau[k] = motor_torque_at<MS>(M, P, k, leg, tgt[k], L.q[k], L.qd[k]);
-    m_sincos(L.q[k], &t.s[k], &t.c[k]);
-  }
+  for (int k = 0; k < 3; ++k) tau[k] = motor_torque_at<MS>(M, P, k, leg, tgt[k], L.q[k], L.qd[k]);
   t.v0 = motion_to_child<0>(B.nu, t.c[0], t.s[0], r0); t.v0.w.x = t.v0.w.x + L.qd[0];
   t.v1 = motion_to_child<1>(t.v0, t.c[1], t.s[1], r1); t.v1.w.y = t.v1.w.y + L.qd[1];
   t.v2 = motion_to_child<1>(t.v1, t.c[2], t.s[2], r2); t.v2.w.y = t.v2.w.y + L.qd[2];
   const SV<T> cb0 = vel_product<0>(t.v0, L.qd[0]), cb1 = vel_product<1>(t.v1, L.qd[1]),
               cb2 = vel_product<1>(t.v2, L.qd[2]);
-  t.g0 = row(B.R, 2);
-  t.g1 = rotT<0>(t.c[0], t.s[0], t.g0);
-  t.g2 = rotT<1>(t.c[1], t.s[1], t.g1);
-  t.g3 = rotT<1>(t.c[2], t.s[2], t.g2);
   t.zf = B.p.z + dot(t.g0, r0) + dot(t.g1, r1) + dot(t.g2, r2) + dot(t.g3, rf);
   t.vf = t.v2.v + cross(t.v2.w, rf);
   t.Fc = contact_force_local(M, T(M.foot_r), t.zf, t.vf, t.g3, &t.mimp);

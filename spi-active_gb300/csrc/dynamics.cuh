@@ -151,6 +151,21 @@ template <class T> SPI_INL V3<T> col(const S3<T>& S, int j) {
   return j == 0 ? v3(S.xx, S.xy, S.xz) : (j == 1 ? v3(S.xy, S.yy, S.yz) : v3(S.xz, S.yz, S.zz));
 }
 
+// Keeps the compiler from fusing an operation across the value's definition: kernels that call the
+// same function on pinned inputs and pin its results get the same bits from it.
+#if defined(__CUDACC__)
+__device__ __forceinline__ void pin(float& x) { asm("" : "+f"(x)); }
+#endif
+template <class T> SPI_INL void pin_device(T& x) { (void)x; }
+SPI_INL void pin_device(float& x) {
+#if defined(__CUDA_ARCH__)
+  pin(x);
+#else
+  (void)x;
+#endif
+}
+template <class T> SPI_INL void pin_device(V3<T>& v) { pin_device(v.x); pin_device(v.y); pin_device(v.z); }
+
 // Active rotation by angle (c, s) about the x (AX = 0) or y (AX = 1) axis, and its transpose.
 template <int AX, class T> SPI_INL V3<T> rot(T c, T s, V3<T> u) {
   if (AX == 0) return v3(u.x, c * u.y - s * u.z, s * u.y + c * u.z);
@@ -994,10 +1009,13 @@ template <class T> SPI_INL LegOut<T> base_terms(const BaseParams<T>& bp, const B
 }
 
 // Base solve and base integration from the total articulated inertia IA and bias force pA at
-// the base, all but the position: d receives the base's displacement. Returns the base
-// acceleration with gravity removed.
-template <class T>
-SPI_INL SV<T> base_solve_step(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B, V3<T>& d) {
+// the base, all but the position: d receives the base's displacement, fac (put_factor) the
+// Cholesky factor of IA. Returns the base acceleration with gravity removed.
+struct NoFactor {
+  template <class T> SPI_INL void put_factor(const T (*)[6], const T*) {}
+};
+template <class T, class FC>
+SPI_INL SV<T> base_solve_step(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B, V3<T>& d, FC& fac) {
   // 6x6 symmetric matrix in (w; v) order, Cholesky L L^T, solve IA a = -pA
   T Mx[6][6];
   Mx[0][0] = IA.A.xx; Mx[1][1] = IA.A.yy; Mx[2][2] = IA.A.zz;
@@ -1025,6 +1043,7 @@ SPI_INL SV<T> base_solve_step(const DevModel& M, const Art<T>& IA, const SV<T>& 
       Mx[i][j] = a * inv;
     }
   }
+  fac.put_factor(Mx, invL);
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
     T a = rhs[i];
@@ -1061,7 +1080,8 @@ SPI_INL SV<T> base_solve_step(const DevModel& M, const Art<T>& IA, const SV<T>& 
 template <class T>
 SPI_INL SV<T> base_solve(const DevModel& M, const Art<T>& IA, const SV<T>& pA, BaseState<T>& B) {
   V3<T> d;
-  const SV<T> a0 = base_solve_step(M, IA, pA, B, d);
+  NoFactor none;
+  const SV<T> a0 = base_solve_step(M, IA, pA, B, d, none);
   B.p = B.p + d;
   return a0;
 }

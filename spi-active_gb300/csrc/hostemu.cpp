@@ -190,6 +190,7 @@ static void substep_vjp(const DevModel& M, const BaseState<T>& B0, const LegStat
     adj::LegTape<T> t;
     T r[3];
     SV<T> fb;
+    adj::leg_pose(B0, L0[leg], t);
     adj::leg_residual<kMotorRuntime>(M, leg, B0, L0[leg], lp[leg], tgt + 3 * leg, a0, qdd[leg], t, r, fb);
     T qb[3] = {T(0), T(0), T(0)}, qdb[3] = {T(0), T(0), T(0)};
     adj::LegParamBar<T> pb = {T(0), T(0), T(0), T(0)};
@@ -331,6 +332,7 @@ static int hostemu_residual(const spi_robot* robot, const double* state, const d
     adj::leg_qdd(W[leg], a0, qdd);
     adj::LegTape<double> t;
     SV<double> fb;
+    adj::leg_pose(B, L[leg], t);
     adj::leg_residual<kMotorRuntime>(M, leg, B, L[leg], lp[leg], tgt + 3 * leg, a0, qdd, t, r, fb);
     adj::add_sv(rb, fb);
     for (int k = 0; k < 3; ++k) out18[3 * leg + k] = r[k];

@@ -68,20 +68,6 @@ template <class S> inline HipLeg<S> hip_leg_constants(const spi_robot& r, int le
   return c;
 }
 
-// Keeps the compiler from fusing an operation across the value's definition: kernels that call the
-// same function on pinned inputs and pin its results get the same bits from it.
-#if defined(__CUDACC__)
-__device__ __forceinline__ void pin(float& x) { asm("" : "+f"(x)); }
-#endif
-template <class T> SPI_INL void pin_device(T& x) { (void)x; }
-SPI_INL void pin_device(float& x) {
-#if defined(__CUDA_ARCH__)
-  pin(x);
-#else
-  (void)x;
-#endif
-}
-
 // Rotation about x by (c, s) of a vector in the y-z plane: active (hip to base) and its transpose.
 template <class T> SPI_INL V3<T> hip_to_base(T c, T s, T x, T y, T z) { return v3(x, c * y - s * z, s * y + c * z); }
 template <class T> SPI_INL V3<T> base_to_hip(T c, T s, V3<T> u) { return v3(u.x, c * u.y + s * u.z, c * u.z - s * u.y); }

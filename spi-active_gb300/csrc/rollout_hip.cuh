@@ -19,7 +19,7 @@
 
 namespace spi {
 
-// pin (leg_hip.cuh) of the composite values handed from one function to the next.
+// pin (dynamics.cuh) of the composite values handed from one function to the next.
 __device__ __forceinline__ void pin3(V3<float>& v) { pin(v.x); pin(v.y); pin(v.z); }
 __device__ __forceinline__ void pin_s3(S3<float>& s) {
   pin(s.xx); pin(s.yy); pin(s.zz); pin(s.xy); pin(s.xz); pin(s.yz);
@@ -157,7 +157,8 @@ __device__ __forceinline__ void substep_hip_lane(const DevModel& M, BaseState<fl
     add_out(sum, o);
   }
   V3<float> d;
-  const SV<float> a0 = base_solve_step(M, sum.I, sum.p, B, d);
+  NoFactor none;
+  const SV<float> a0 = base_solve_step(M, sum.I, sum.p, B, d, none);
   carry_add(B.p, pe, d);
   pin(B);
 #pragma unroll 1
@@ -336,7 +337,8 @@ struct TeamRollout {
     pin(W);
     const LegOut<float> sum = team_sum(share, base, o);
     V3<float> d;
-    const SV<float> a0 = base_solve_step(M, sum.I, sum.p, B, d);
+    NoFactor none;
+    const SV<float> a0 = base_solve_step(M, sum.I, sum.p, B, d, none);
     carry_add(B.p, pe, d);
     pin(B);
     joint_step(M, a0, W, L, qe);

@@ -1,0 +1,39 @@
+"""The adjoint over its batches and segments: horizons past a segment of 50 control steps, and batches of
+(theta, window group) pairs past its scratch."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import oracle_windows, random_theta
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,W", [(50, 3), (51, 9), (104, 2)])
+def test_segments_agree_with_forward_mode(built, H, W):
+    """Within the 1e-3 the adjoint is held to everywhere, of the forward-mode gradient."""
+    from spi_gb300.engine import Engine
+    from spi_gb300.sensitivity import adjoint, tangent_gradient
+    _, init, actions, target = oracle_windows(31, n_traj=1, T=W + H + 1, H=H)
+    e = Engine()
+    e.load_windows(*(torch.from_numpy(a[:W]) for a in (init, actions, target)))
+    th = torch.from_numpy(random_theta(np.random.default_rng(3), 3).astype(np.float32))
+    cost, grad = adjoint(e, th)
+    ref_cost, ref = tangent_gradient(e, th)
+    assert torch.allclose(cost, ref_cost, rtol=1e-4)
+    assert (torch.linalg.norm(grad - ref, dim=1) <= 1e-3 * torch.linalg.norm(ref, dim=1)).all()
+
+
+def test_batches_do_not_change_a_row(built):
+    """4 GB of kept substeps hold some 3,600 pairs at H = 50: 150 theta x 32 groups take two batches."""
+    from spi_gb300.engine import Engine
+    from spi_gb300.sensitivity import adjoint
+    _, init, actions, target = oracle_windows(32, n_traj=4, T=120, H=50)
+    e = Engine()
+    init, actions, target = (torch.from_numpy(a).repeat(*([4] + [1] * (a.ndim - 1)))[:256] for a in (init, actions, target))
+    e.load_windows(init, actions, target)
+    th = torch.from_numpy(random_theta(np.random.default_rng(4), 150).astype(np.float32))
+    cost, grad = adjoint(e, th)
+    for rows in (slice(0, 3), slice(70, 90), slice(149, 150)):
+        c, g = adjoint(e, th[rows])
+        assert torch.equal(c, cost[rows]) and torch.equal(g, grad[rows])
