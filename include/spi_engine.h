@@ -138,7 +138,10 @@ int spi_set_kernel_layout(spi_engine* e, int layout);
 
 /* Roll every (theta, window) pair H control steps and reduce the windowed cost. Async. */
 int spi_run(spi_engine* e);
-/* Same, also writing every control step's state to trace, device [N][W][H][37]. */
+/* spi_set_theta, spi_run and spi_read_costs in one call: theta device [N][13], comp device [N][9] and
+ * cost device [N] (either may be NULL). The same results, without the copies in between. Async. */
+int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* cost);
+/* spi_run, also writing every control step's state to trace, device [N][W][H][37]. */
 int spi_run_trace(spi_engine* e, float* trace);
 
 /* Advance caller-owned states in place: state device [B][37] (world frame, the reference's

@@ -12,6 +12,7 @@
 #include "model.h"
 #include "rollout.cuh"
 #include "rollout_block.cuh"
+#include "windows.cuh"
 
 using namespace spi;
 
@@ -33,24 +34,33 @@ int cuda_error(cudaError_t e, const char* what) {
 
 namespace {
 
-__global__ void rows_to_soa(const float* __restrict__ src, float* __restrict__ dst, int W, int F) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)W * F) return;
-  const int w = (int)(i / F), f = (int)(i % F);
-  dst[(size_t)f * W + w] = src[i];
+// finalize_costs for spi_evaluate, in the same launch to the caller's outputs and with the theta batch
+// kept as the engine's own: the call has no copies to wait for.
+__global__ void finalize_evaluate(const float* __restrict__ partial, int N, int G, float norm, int mode, float w0,
+                                  float w1, float w2, float w3, float w4, float w5, const float* __restrict__ theta,
+                                  float* __restrict__ own_theta, float* __restrict__ own_comp,
+                                  float* __restrict__ own_cost, float* __restrict__ comp, float* __restrict__ cost) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const float w[6] = {w0, w1, w2, w3, w4, w5};
+  finalize_one(partial, n, G, norm, mode, w, own_comp, own_cost);
+#pragma unroll
+  for (int i = 0; i < SPI_THETA_DIM; ++i) own_theta[(size_t)n * SPI_THETA_DIM + i] = theta[(size_t)n * SPI_THETA_DIM + i];
+  if (comp) {
+#pragma unroll
+    for (int k = 0; k < SPI_N_COMP; ++k) comp[(size_t)n * SPI_N_COMP + k] = own_comp[(size_t)n * SPI_N_COMP + k];
+  }
+  if (cost) cost[n] = own_cost[n];
 }
-__global__ void actions_to_hw(const float* __restrict__ src, float* __restrict__ dst, int W, int H) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)W * H * 12) return;
-  const int j = (int)(i % 12);
-  const long long wh = i / 12;
-  const int h = (int)(wh % H), w = (int)(wh / H);
-  dst[((size_t)h * W + w) * 12 + j] = src[i];
+
+// The buffers of a run over the engine's theta batch.
+int reserve_run(spi_engine* e, int G) {
+  int rc = e->partial.reserve((size_t)e->N * G * SPI_N_COMP * sizeof(float));
+  if (!rc) rc = e->comp.reserve((size_t)e->N * SPI_N_COMP * sizeof(float));
+  if (!rc) rc = e->cost.reserve((size_t)e->N * sizeof(float));
+  return rc ? rc : refresh_after_realloc(e);
 }
-__global__ void fill_f32(float* p, float v, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
+
 }  // namespace
 
 int spi::run_impl(spi_engine* e, float* trace) {
@@ -58,13 +68,8 @@ int spi::run_impl(spi_engine* e, float* trace) {
   if (e->W <= 0 || e->H <= 0) return set_error(SPI_ESTATE, "spi_run before spi_load_windows");
   if (e->N <= 0) return set_error(SPI_ESTATE, "spi_run before spi_set_theta");
   const int G = (e->W + 7) / 8;
-  int rc = e->partial.reserve((size_t)e->N * G * SPI_N_COMP * sizeof(float));
+  int rc = reserve_run(e, G);
   if (rc) return rc;
-  rc = e->comp.reserve((size_t)e->N * SPI_N_COMP * sizeof(float));
-  if (rc) return rc;
-  rc = e->cost.reserve((size_t)e->N * sizeof(float));
-  if (rc) return rc;
-  if ((rc = refresh_after_realloc(e))) return rc;
   WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
   const long long warps = (long long)e->N * G;
   const unsigned grid = blocks_for(warps, 4);
@@ -181,15 +186,8 @@ int spi_load_windows(spi_engine* e, const float* init, const float* actions, con
   if ((rc = e->act.reserve((size_t)W * H * 12 * 4))) return rc;
   if ((rc = e->weight.reserve((size_t)W * 4))) return rc;
   if ((rc = refresh_after_realloc(e))) return rc;
-  const long long ns = (long long)W * SPI_STATE_DIM;
-  rows_to_soa<<<blocks_for(ns, 256), 256, 0, e->stream>>>(init, e->init.f(), W, SPI_STATE_DIM);
-  rows_to_soa<<<blocks_for(ns, 256), 256, 0, e->stream>>>(target, e->tgt.f(), W, SPI_STATE_DIM);
-  actions_to_hw<<<blocks_for((long long)W * H * 12, 256), 256, 0, e->stream>>>(actions, e->act.f(), W, H);
-  if (weight)
-    cudaMemcpyAsync(e->weight.p, weight, (size_t)W * 4, cudaMemcpyDeviceToDevice, e->stream);
-  else
-    fill_f32<<<blocks_for(W, 256), 256, 0, e->stream>>>(e->weight.f(), 1.0f, W);
-  cudaError_t ce = cudaGetLastError();
+  const cudaError_t ce = pack_windows(init, actions, target, weight, W, H, e->init.f(), e->act.f(), e->tgt.f(),
+                                      e->weight.f(), e->stream);
   if (ce != cudaSuccess) return cuda_error(ce, "spi_load_windows");
   e->W = W;
   e->H = H;
@@ -252,6 +250,36 @@ int spi_set_cost(spi_engine* e, int mode, const float* sq_weights) {
 }
 
 int spi_run(spi_engine* e) { return run_impl(e, nullptr); }
+
+int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* cost) {
+  if (!e || !theta) return set_error(SPI_EINVAL, "spi_evaluate: null argument");
+  if (N <= 0) return set_error(SPI_EINVAL, "spi_evaluate: N=%d must be > 0", N);
+  if (e->W <= 0 || e->H <= 0) return set_error(SPI_ESTATE, "spi_evaluate before spi_load_windows");
+  if (e->layout != SPI_LAYOUT_LANE) {
+    int rc = spi_set_theta(e, theta, N);
+    if (!rc) rc = run_impl(e, nullptr);
+    return rc ? rc : spi_read_costs(e, comp, cost);
+  }
+  const int G = (e->W + 7) / 8;
+  int rc = e->theta.reserve((size_t)N * SPI_THETA_DIM * 4);
+  if (rc) return rc;
+  e->N = N;
+  e->population = false;
+  e->ran = false;
+  if ((rc = reserve_run(e, G))) return rc;
+  const WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
+  const EvalArgs a{win, theta, e->partial.f(), N, G, (unsigned long long*)e->bad.p};
+  cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);
+  if (ce != cudaSuccess) return cuda_error(ce, "spi_evaluate: rollout launch");
+  const float* w = e->sq_w;
+  finalize_evaluate<<<blocks_for(N, 128), 128, 0, e->stream>>>(e->partial.f(), N, G, e->norm, e->cost_mode, w[0], w[1],
+                                                               w[2], w[3], w[4], w[5], theta, e->theta.f(), e->comp.f(),
+                                                               e->cost.f(), comp, cost);
+  ce = cudaGetLastError();
+  if (ce != cudaSuccess) return cuda_error(ce, "spi_evaluate: finalize launch");
+  e->ran = true;
+  return SPI_OK;
+}
 
 int spi_run_trace(spi_engine* e, float* trace) {
   if (!trace) return set_error(SPI_EINVAL, "spi_run_trace: null trace");

@@ -21,6 +21,7 @@
 #include "items.h"
 #include "model.h"
 #include "rollout.cuh"
+#include "windows.cuh"
 
 using namespace spi;
 
@@ -45,24 +46,6 @@ struct SlotHost {
   cudaEvent_t done = nullptr;
   SlotDesc desc;
 };
-
-__global__ void srv_rows_to_soa(const float* __restrict__ src, float* __restrict__ dst, int W, int F) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)W * F) return;
-  dst[(size_t)(i % F) * W + (i / F)] = src[i];
-}
-__global__ void srv_actions_to_hw(const float* __restrict__ src, float* __restrict__ dst, int W, int H) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)W * H * 12) return;
-  const int j = (int)(i % 12);
-  const long long wh = i / 12;
-  const int h = (int)(wh % H), w = (int)(wh / H);
-  dst[((size_t)h * W + w) * 12 + j] = src[i];
-}
-__global__ void srv_fill(float* p, float v, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
 
 __global__ void server_finalize_kernel(const SlotDesc* __restrict__ slots, const int* __restrict__ rounds, int round,
                                        int mode, float w0, float w1, float w2, float w3, float w4, float w5) {
@@ -437,15 +420,8 @@ int spi_server_submit(spi_server* s, const spi_job* job, int32_t* slot_out) {
   d.G = (job->W + 7) / 8;
   d.norm = job->norm > 0.f ? job->norm : (float)job->W;
   d.active = 1;
-  const long long ns = (long long)job->W * SPI_STATE_DIM;
-  srv_rows_to_soa<<<(unsigned)((ns + 255) / 256), 256, 0, s->stream>>>(job->init, (float*)d.win.init, job->W, SPI_STATE_DIM);
-  srv_rows_to_soa<<<(unsigned)((ns + 255) / 256), 256, 0, s->stream>>>(job->target, (float*)d.win.tgt, job->W, SPI_STATE_DIM);
-  const long long na = (long long)job->W * job->H * 12;
-  srv_actions_to_hw<<<(unsigned)((na + 255) / 256), 256, 0, s->stream>>>(job->actions, (float*)d.win.act, job->W, job->H);
-  if (job->weight)
-    ce = cudaMemcpyAsync((void*)d.win.weight, job->weight, (size_t)job->W * 4, cudaMemcpyDeviceToDevice, s->stream);
-  else
-    srv_fill<<<(job->W + 255) / 256, 256, 0, s->stream>>>((float*)d.win.weight, 1.0f, job->W);
+  ce = pack_windows(job->init, job->actions, job->target, job->weight, job->W, job->H, (float*)d.win.init,
+                    (float*)d.win.act, (float*)d.win.tgt, (float*)d.win.weight, s->stream);
   memcpy(h.nominal, c.nominal, sizeof(h.nominal));
   memcpy(h.best_theta, c.nominal, sizeof(h.best_theta));
   h.best_cost = INFINITY;

@@ -36,6 +36,7 @@ ENGINE_API = {
     "spi_set_theta": (c_int, [c_void_p, c_void_p, c_int]),
     "spi_set_cost": (c_int, [c_void_p, c_int, POINTER(c_float)]),
     "spi_run": (c_int, [c_void_p]),
+    "spi_evaluate": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
     "spi_set_kernel_config": (c_int, [c_void_p, c_int]),
     "spi_set_kernel_layout": (c_int, [c_void_p, c_int]),
     "spi_run_trace": (c_int, [c_void_p, c_void_p]),

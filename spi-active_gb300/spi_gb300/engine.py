@@ -116,10 +116,19 @@ class Engine:
 
     def evaluate(self, theta, trace=False):
         """Mean error components [N,9], scalar cost [N] (and the trace [N,W,H,37])."""
-        self.set_theta(theta)
-        tr = self.run(trace=trace)
-        comp, cost = self.read()
-        return (comp, cost, tr) if trace else (comp, cost)
+        if trace:
+            self.set_theta(theta)
+            tr = self.run(trace=True)
+            comp, cost = self.read()
+            return comp, cost, tr
+        theta = _f32(theta, (int(theta.shape[0]), THETA_DIM), "theta", self.device)
+        N = theta.shape[0]
+        comp = torch.empty((N, N_COMP), device=self.device)
+        cost = torch.empty((N,), device=self.device)
+        _lib.check(self.lib.spi_evaluate(self._h, theta.data_ptr(), N, comp.data_ptr(), cost.data_ptr()))
+        self._theta = theta
+        self.N = N
+        return comp, cost
 
 
 def probe_fp32_peak() -> float:

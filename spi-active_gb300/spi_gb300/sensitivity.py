@@ -99,7 +99,7 @@ class WindowCost(torch.autograd.Function):
         _, cost = engine.evaluate(th)
         ctx.engine = engine
         ctx.save_for_backward(th)
-        return cost.clone()
+        return cost
 
     @staticmethod
     def backward(ctx, g):
