@@ -232,13 +232,27 @@ template <class T> struct LegTape {
   V3<T> vf, Fc;                      // foot velocity and contact force (calf frame)
 };
 
+// a b + c d, c d rounded first. The contacts' branches (on or off, stick or slip) turn on the last bits of the
+// foot's height and velocity: left to the compiler, which product of a rotation is fused varies with the code
+// around it, and with it the branch, hence the gradient, of the few contacts at an edge.
+template <class T> SPI_INL T mul_add2(T a, T b, T c, T d) { return a * b + c * d; }
+#ifdef __CUDA_ARCH__
+template <> SPI_INL float mul_add2<float>(float a, float b, float c, float d) {
+  return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+#endif
+
 // The pose's part of the tape: joint sines and cosines, and the world vertical down the leg.
 template <class T> SPI_INL void leg_pose(const BaseState<T>& B, const LegState<T>& L, LegTape<T>& t) {
   for (int k = 0; k < 3; ++k) m_sincos(L.q[k], &t.s[k], &t.c[k]);
   t.g0 = row(B.R, 2);
-  t.g1 = rotT<0>(t.c[0], t.s[0], t.g0);
-  t.g2 = rotT<1>(t.c[1], t.s[1], t.g1);
-  t.g3 = rotT<1>(t.c[2], t.s[2], t.g2);
+  t.g1 = v3(t.g0.x, mul_add2(t.c[0], t.g0.y, t.s[0], t.g0.z), mul_add2(t.c[0], t.g0.z, -t.s[0], t.g0.y));
+  t.g2 = v3(mul_add2(t.c[1], t.g1.x, -t.s[1], t.g1.z), t.g1.y, mul_add2(t.s[1], t.g1.x, t.c[1], t.g1.z));
+  t.g3 = v3(mul_add2(t.c[2], t.g2.x, -t.s[2], t.g2.z), t.g2.y, mul_add2(t.s[2], t.g2.x, t.c[2], t.g2.z));
+}
+// An angular velocity carried across a thigh or calf joint (rotT<1>).
+template <class T> SPI_INL V3<T> turn_y(T c, T s, V3<T> w) {
+  return v3(mul_add2(c, w.x, -s, w.z), w.y, mul_add2(c, w.z, s, w.x));
 }
 
 // r[k]: joint k's residual f_k . S_k + arm qdd_k - tau_k; fb: the leg's force on the base
@@ -253,8 +267,12 @@ SPI_INL void leg_residual(const DevModel& M, int leg, const BaseState<T>& B, con
   T tau[3];
   for (int k = 0; k < 3; ++k) tau[k] = motor_torque_at<MS>(M, P, k, leg, tgt[k], L.q[k], L.qd[k]);
   t.v0 = motion_to_child<0>(B.nu, t.c[0], t.s[0], r0); t.v0.w.x = t.v0.w.x + L.qd[0];
-  t.v1 = motion_to_child<1>(t.v0, t.c[1], t.s[1], r1); t.v1.w.y = t.v1.w.y + L.qd[1];
-  t.v2 = motion_to_child<1>(t.v1, t.c[2], t.s[2], r2); t.v2.w.y = t.v2.w.y + L.qd[2];
+  t.v1 = motion_to_child<1>(t.v0, t.c[1], t.s[1], r1);
+  t.v1.w = turn_y(t.c[1], t.s[1], t.v0.w);
+  t.v1.w.y = t.v1.w.y + L.qd[1];
+  t.v2 = motion_to_child<1>(t.v1, t.c[2], t.s[2], r2);
+  t.v2.w = turn_y(t.c[2], t.s[2], t.v1.w);
+  t.v2.w.y = t.v2.w.y + L.qd[2];
   const SV<T> cb0 = vel_product<0>(t.v0, L.qd[0]), cb1 = vel_product<1>(t.v1, L.qd[1]),
               cb2 = vel_product<1>(t.v2, L.qd[2]);
   t.zf = B.p.z + dot(t.g0, r0) + dot(t.g1, r1) + dot(t.g2, r2) + dot(t.g3, rf);
