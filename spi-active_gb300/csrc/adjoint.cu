@@ -22,6 +22,7 @@
 
 #include "adjoint.cuh"
 #include "engine_impl.h"
+#include "kept.cuh"
 #include "rollout.cuh"
 
 using namespace spi;
@@ -30,55 +31,7 @@ namespace {
 
 constexpr int kSegSteps = 50;                       // control steps between checkpoints
 constexpr size_t kScratch = (size_t)4 << 30;        // bytes of kept substeps
-constexpr int kLegFields = 9;                       // 16-byte fields per lane and kept substep
-constexpr int kBaseFields = 10;                     // and per rollout
-constexpr size_t kPairBytes = 32 * 16 * kLegFields + 8 * 16 * kBaseFields;   // a warp's, per substep
-
-// Cholesky factor of a 6x6 symmetric positive definite matrix: the strict lower triangle by rows and
-// the inverse diagonal.
-struct Factor6 {
-  float l[15], inv[6];
-  __device__ __forceinline__ void put_factor(const float (*Mx)[6], const float* invL) {
-    int k = 0;
-#pragma unroll
-    for (int i = 1; i < 6; ++i)
-#pragma unroll
-      for (int j = 0; j < i; ++j) l[k++] = Mx[i][j];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) inv[i] = invL[i];
-  }
-  __device__ __forceinline__ SV<float> solve(const SV<float>& b) const {
-    float x[6] = {b.w.x, b.w.y, b.w.z, b.v.x, b.v.y, b.v.z};
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      float a = x[i];
-#pragma unroll
-      for (int k = 0; k < i; ++k) a = a - l[i * (i - 1) / 2 + k] * x[k];
-      x[i] = a * inv[i];
-    }
-#pragma unroll
-    for (int i = 5; i >= 0; --i) {
-      float a = x[i];
-#pragma unroll
-      for (int k = i + 1; k < 6; ++k) a = a - l[k * (k - 1) / 2 + i] * x[k];
-      x[i] = a * inv[i];
-    }
-    SV<float> r;
-    r.w = v3(x[0], x[1], x[2]);
-    r.v = v3(x[3], x[4], x[5]);
-    return r;
-  }
-};
-
-// A warp's kept substeps: leg fields [slot][field][lane], base fields [slot][field][rollout].
-struct Kept {
-  float4* leg;     // at this lane
-  float4* base;    // at this lane's rollout
-  size_t leg_slot, base_slot;   // 16-byte fields from one slot to the next (of the whole batch)
-  size_t leg_field, base_field;
-  __device__ __forceinline__ float4* leg_at(int slot, int f) const { return leg + slot * leg_slot + f * leg_field; }
-  __device__ __forceinline__ float4* base_at(int slot, int f) const { return base + slot * base_slot + f * base_field; }
-};
+constexpr size_t kPairBytes = 8 * kKeptBytes;       // a warp's eight rollouts', per substep
 
 // Phase A's work record to its parking slot (for phase C) and to the kept substep.
 struct KeptWork {
@@ -93,58 +46,6 @@ struct KeptWork {
   }
   __device__ __forceinline__ void put_diag(float a, float b, float c) { diag[0] = a; diag[1] = b; diag[2] = c; }
 };
-
-__device__ __forceinline__ void keep_state(const Kept& k, int slot, int leg, const BaseState<float>& B) {
-  if (leg != 0) return;
-  __stcs(k.base_at(slot, 0), make_float4(B.p.x, B.p.y, B.p.z, B.qx));
-  __stcs(k.base_at(slot, 1), make_float4(B.qy, B.qz, B.qw, B.nu.w.x));
-  __stcs(k.base_at(slot, 2), make_float4(B.nu.w.y, B.nu.w.z, B.nu.v.x, B.nu.v.y));
-}
-__device__ __forceinline__ void keep_legs(const Kept& k, int slot, const float d[3], const LegState<float>& L) {
-  __stcs(k.leg_at(slot, 6), make_float4(d[0], d[1], d[2], L.q[0]));
-  __stcs(k.leg_at(slot, 7), make_float4(L.q[1], L.q[2], L.qd[0], L.qd[1]));
-  __stcs(k.leg_at(slot, 8), make_float4(L.qd[2], 0.f, 0.f, 0.f));
-}
-// The state and, for WORK, the factorisations of a kept substep.
-template <bool WORK>
-__device__ __forceinline__ void load_kept(const Kept& k, int slot, BaseState<float>& B, LegState<float>& L,
-                                          adj::SolveWork<float>& W, Factor6& fac, SV<float>& a0) {
-  const float4 b0 = __ldcs(k.base_at(slot, 0)), b1 = __ldcs(k.base_at(slot, 1)), b2 = __ldcs(k.base_at(slot, 2)),
-               b3 = __ldcs(k.base_at(slot, 3));
-  const float4 l6 = __ldcs(k.leg_at(slot, 6)), l7 = __ldcs(k.leg_at(slot, 7)), l8 = __ldcs(k.leg_at(slot, 8));
-  if (WORK) {
-    float l[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float4 u = __ldcs(k.leg_at(slot, 2 * c)), v = __ldcs(k.leg_at(slot, 2 * c + 1));
-      W.Kp[c].w = v3(u.x, u.y, u.z);
-      W.Kp[c].v = v3(u.w, v.x, v.y);
-      W.y[c] = v.z;
-      l[c] = v.w;
-    }
-    W.l10 = l[0]; W.l20 = l[1]; W.l21 = l[2];
-    W.i[0] = l6.x; W.i[1] = l6.y; W.i[2] = l6.z;
-    float v[24];
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      const float4 u = __ldcs(k.base_at(slot, 4 + f));
-      v[4 * f] = u.x; v[4 * f + 1] = u.y; v[4 * f + 2] = u.z; v[4 * f + 3] = u.w;
-    }
-    a0.w = v3(b3.y, b3.z, b3.w);
-    a0.v = v3(v[0], v[1], v[2]);
-#pragma unroll
-    for (int i = 0; i < 15; ++i) fac.l[i] = v[3 + i];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) fac.inv[i] = v[18 + i];
-  }
-  B.p = v3(b0.x, b0.y, b0.z);
-  B.qx = b0.w; B.qy = b1.x; B.qz = b1.y; B.qw = b1.z;
-  B.nu.w = v3(b1.w, b2.x, b2.y);
-  B.nu.v = v3(b2.z, b2.w, b3.x);
-  B.R = quat_to_R(B.qx, B.qy, B.qz, B.qw);
-  L.q[0] = l6.w; L.q[1] = l7.x; L.q[2] = l7.y;
-  L.qd[0] = l7.z; L.qd[1] = l7.w; L.qd[2] = l8.x;
-}
 
 // substep (rollout.cuh), keeping the state it starts from and its factorisations in `slot`.
 __device__ __forceinline__ void substep_kept(const DevModel& M, int leg, BaseState<float>& B, LegState<float>& L,
@@ -164,15 +65,7 @@ __device__ __forceinline__ void substep_kept(const DevModel& M, int leg, BaseSta
   Factor6 fac;
   const SV<float> a0 = base_solve_step(M, IA, pA, B, d, fac);
   B.p = B.p + d;
-  if (leg == 0) {
-    __stcs(k.base_at(slot, 3), make_float4(nuz, a0.w.x, a0.w.y, a0.w.z));
-    __stcs(k.base_at(slot, 4), make_float4(a0.v.x, a0.v.y, a0.v.z, fac.l[0]));
-#pragma unroll
-    for (int f = 0; f < 3; ++f)
-      __stcs(k.base_at(slot, 5 + f), make_float4(fac.l[4 * f + 1], fac.l[4 * f + 2], fac.l[4 * f + 3], fac.l[4 * f + 4]));
-    __stcs(k.base_at(slot, 8), make_float4(fac.l[13], fac.l[14], fac.inv[0], fac.inv[1]));
-    __stcs(k.base_at(slot, 9), make_float4(fac.inv[2], fac.inv[3], fac.inv[4], fac.inv[5]));
-  }
+  keep_solve(k, slot, leg, nuz, a0, fac);
   LegWork<float> lw;
   unpark_legwork(lw, lw_smem + threadIdx.x, 128);
   phase_c(M, leg, a0, lw, L);
@@ -278,8 +171,7 @@ struct AdjArgs {
   unsigned long long* n_bad;
 
   __device__ __forceinline__ Kept kept(long long local, int lane) const {
-    return Kept{legs + local * 32 + lane, base + local * 8 + (lane >> 2), (size_t)pairs * 32 * kLegFields,
-                (size_t)pairs * 8 * kBaseFields, (size_t)pairs * 32, (size_t)pairs * 8};
+    return Kept::of(legs, base, (size_t)pairs * 8, (size_t)local * 8 + (lane >> 2), lane & 3);
   }
   __device__ __forceinline__ Kept checkpoints(long long local, int lane) const {
     Kept k = kept(local, lane);

@@ -20,6 +20,7 @@ struct Df {
   SPI_INL Df(float x, float dx) : v(x), d(dx) {}
 };
 
+SPI_INL float scalar_value(Df x) { return x.v; }
 SPI_INL Df operator+(Df a, Df b) { return Df(a.v + b.v, a.d + b.d); }
 SPI_INL Df operator-(Df a, Df b) { return Df(a.v - b.v, a.d - b.d); }
 SPI_INL Df operator*(Df a, Df b) { return Df(a.v * b.v, a.d * b.v + a.v * b.d); }

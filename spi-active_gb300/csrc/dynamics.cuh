@@ -580,6 +580,12 @@ SPI_INL auto put_diag_if(WK& w, T i0, T i1, T i2, int) -> decltype(w.put_diag(i0
   w.put_diag(i0, i1, i2);
 }
 template <class WK, class T> SPI_INL void put_diag_if(WK&, T, T, T, long) {}
+// Likewise put_contact: the foot's height and its contact's branch (contact_force_local).
+template <class WK, class T>
+SPI_INL auto put_contact_if(WK& w, T zf, const T* branch, int) -> decltype(w.put_contact(zf, branch), void()) {
+  w.put_contact(zf, branch);
+}
+template <class WK, class T> SPI_INL void put_contact_if(WK&, T, const T*, long) {}
 
 template <class T> SPI_INL M3<T> quat_to_R(T x, T y, T z, T w) {
   M3<T> R;
@@ -636,8 +642,10 @@ template <class T> SPI_INL V3<T> contact_force(const DevModel& M, T radius, T z,
 // contact_force evaluated in the frame of the contact point's body: n is the world vertical
 // there (unit), v the point's velocity there. The tangential velocity is v - (n.v) n, whose norm
 // is the world-horizontal speed; returns the force in that frame with the implicit point mass's
-// share of the gravity shift (mimp g along n) included.
-template <class T> SPI_INL V3<T> contact_force_local(const DevModel& M, T radius, T z, V3<T> v, V3<T> n, T* mimp) {
+// share of the gravity shift (mimp g along n) included. branch (optional): receives the normal
+// force and the tangential scale, which tell the branch taken (0: off; the model's ct: sticking).
+template <class T>
+SPI_INL V3<T> contact_force_local(const DevModel& M, T radius, T z, V3<T> v, V3<T> n, T* mimp, T* branch = nullptr) {
   const T vz = dot(n, v);
   const V3<T> vt = v3(v.x - vz * n.x, v.y - vz * n.y, v.z - vz * n.z);
   T pen = radius - z;
@@ -647,6 +655,10 @@ template <class T> SPI_INL V3<T> contact_force_local(const DevModel& M, T radius
   T lim = T(M.mu) * fn;
   T scale = m_sel(T(M.ct) * vtn <= lim, T(M.ct), lim / vtn);
   *mimp = m_mul2_c(s, M.dt, M.imp_c, M.dt_imp_c);
+  if (branch) {
+    branch[0] = fn;
+    branch[1] = scale;
+  }
   const T fz = fn + *mimp * T(M.g);
   return v3(fz * n.x - scale * vt.x, fz * n.y - scale * vt.y, fz * n.z - scale * vt.z);
 }
@@ -875,9 +887,10 @@ SPI_INL void phase_a_core(const DevModel& M, int leg, const BaseState<T>& B, con
   const V3<T> g2 = rotT<1>(C[1], S[1], g1);
   const V3<T> g3 = rotT<1>(C[2], S[2], g2);
   const T zf = B.p.z + g0.x * r0.x + g0.y * r0.y + g1.y * r1.y + g2.z * r2.z + g3.z * fz;
-  T mimp;
+  T mimp, branch[2];
   const V3<T> Fc = contact_force_local(M, T(M.foot_r), zf, v3(v2.v.x + v2.w.y * fz, v2.v.y - v2.w.x * fz, v2.v.z),
-                                       g3, &mimp);
+                                       g3, &mimp, branch);
+  put_contact_if(W, zf, branch, 0);
   // composite inertias: calf (+ the contact's implicit point mass at the foot) -> thigh -> hip
   const RI<T> Ical = lc_ri<T>(lc, 2);
   RI<T> Rc2 = Ical;

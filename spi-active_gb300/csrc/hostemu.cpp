@@ -15,6 +15,7 @@
 #include "aba_reference.h"
 #include "adjoint.cuh"
 #include "model.h"
+#include "tangent.cuh"
 
 namespace spi {
 
@@ -304,6 +305,57 @@ static int hostemu_grad(const spi_robot* robot, const double* init, const double
   return SPI_OK;
 }
 
+// The tangent of one substep (tangent.cuh) along dB / dL / theta slot k, legs in a loop; B / L are advanced too.
+template <class T>
+static void substep_tan(const DevModel& M, BaseState<T>& B, LegState<T> L[4], const BaseParams<T>& bp, const LegParams<T> lp[4],
+                        const T* th, int k, const T tgt[12], tng::BaseTan<T>& dB, tng::LegTan<T> dL[4]) {
+  adj::SolveWork<T> W[4];
+  LegOut<T> sum = base_terms(bp, B);
+  const bool corners = corners_may_touch(M, B);
+  for (int leg = 0; leg < 4; ++leg) phase_a_into(M, leg, B, L[leg], lp[leg], tgt + 3 * leg, W[leg], sum, corners);
+  const Art<T> IA = sum.I;
+  const BaseState<T> B0 = B;
+  const SV<T> a0 = base_solve(M, sum.I, sum.p, B);
+  tng::ParamTan<T> dP;
+  tng::base_params_tan(M, th, k, dP.m, dP.h, dP.Io);
+  SV<T> drb = tng::base_residual_tan(bp, B0, a0, dB, dP);
+  T lam[4][3];
+  for (int leg = 0; leg < 4; ++leg) {
+    T qdd[3], r[3], dr[3];
+    adj::leg_qdd(W[leg], a0, qdd);
+    adj::LegTape<T> t;
+    SV<T> fb, dfb;
+    adj::leg_pose(B0, L[leg], t);
+    adj::leg_residual<kMotorRuntime>(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, a0, qdd, t, r, fb);
+    const int s0 = leg >= 2 ? 9 : 5;
+    dP.kps = T(k == s0); dP.fc = T(k == s0 + 1); dP.arm = T(k == s0 + 2); dP.ts = T(k == s0 + 3);
+    const V3<T> vt = t.vf + (-dot(t.g3, t.vf)) * t.g3;
+    const T pen = T(M.foot_r) - t.zf;
+    const T fn = m_fmax(T(0), T(M.k) * pen - T(M.c) * m_clamp(pen * T(M.ramp_inv), T(0), T(1)) * dot(t.g3, t.vf));
+    const tng::ContactBranch br = {fn > T(0), T(M.ct) * m_sqrt(dot(vt, vt)) <= T(M.mu) * fn};
+    tng::leg_residual_tan(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, qdd, t, t.zf, br, dB, dL[leg], dP, dr, dfb);
+    adj::add_sv(drb, dfb);
+    if (corners)
+      for (int j = 0; j < 2; ++j)
+        adj::add_sv(drb, tng::corner_residual_tan(M, B0, lc_corner<T>(M.legc[leg], j), a0, dB));
+    for (int i = 0; i < 3; ++i) lam[leg][i] = -dr[i];
+  }
+  T z[4][3];
+  SV<T> rhs = adj::sub_sv(adj::zsv<T>(), drb);
+  for (int leg = 0; leg < 4; ++leg) rhs = adj::sub_sv(rhs, adj::leg_solve_down(W[leg], lam[leg], z[leg]));
+  const SV<T> da0 = adj::art_solve(IA, rhs);
+  tng::base_integrate_tan(M, B0, B, da0, dB);
+  for (int leg = 0; leg < 4; ++leg) {
+    T dqdd[3];
+    adj::leg_solve_up(W[leg], z[leg], da0, dqdd);
+    for (int i = 0; i < 3; ++i) {
+      dL[leg].qd[i] = dL[leg].qd[i] + T(M.dt) * dqdd[i];
+      dL[leg].q[i] = dL[leg].q[i] + T(M.dt) * dL[leg].qd[i];
+    }
+    phase_c(M, leg, a0, W[leg], L[leg]);
+  }
+}
+
 // The residual r(x, theta, a) at the accelerations the forward substep computes: [4][3] joint
 // residuals and the base's 6 (near zero up to rounding when the residual is the forward's model).
 static int hostemu_residual(const spi_robot* robot, const double* state, const double* theta, const double* act12,
@@ -463,6 +515,36 @@ int spi_hostemu_count_ops_aba(const spi_robot* robot, const double* state, const
 int spi_hostemu_grad(const spi_robot* robot, const double* init, const double* actions, const double* theta,
                      const double* target, const double* qw, int mode, int nb, int H, double* cost, double* grad) {
   return hostemu_grad<double>(robot, init, actions, theta, target, qw, mode, nb, H, cost, grad);
+}
+// Final state [37] and its derivative in theta slot k, d [37], by the substep tangents (FP64).
+int spi_hostemu_tangent(const spi_robot* robot, const double* init, const double* actions, const double* theta, int k,
+                        int H, double* state, double* tangent) {
+  DevModel M;
+  const char* why = "";
+  int rc = build_dev_model(*robot, &M, &why);
+  if (rc) return rc;
+  BaseState<double> B;
+  LegState<double> L[4];
+  BaseParams<double> bp;
+  LegParams<double> lp[4];
+  load_rollout(M, init, theta, B, L, bp, lp);
+  tng::BaseTan<double> dB = tng::zero_base_tan<double>();
+  tng::LegTan<double> dL[4] = {};
+  for (int h = 0; h < H; ++h) {
+    double tgt[12];
+    for (int j = 0; j < 12; ++j) tgt[j] = joint_target(M, j % 3, j / 3, actions[h * 12 + j]);
+    for (int s = 0; s < M.decimation; ++s) substep_tan(M, B, L, bp, lp, theta, k, tgt, dB, dL);
+  }
+  base_to_world(B, state);
+  tng::base_to_world_tan(B, dB, tangent);
+  for (int leg = 0; leg < 4; ++leg)
+    for (int i = 0; i < 3; ++i) {
+      state[13 + 3 * leg + i] = L[leg].q[i];
+      state[25 + 3 * leg + i] = L[leg].qd[i];
+      tangent[13 + 3 * leg + i] = dL[leg].q[i];
+      tangent[25 + 3 * leg + i] = dL[leg].qd[i];
+    }
+  return SPI_OK;
 }
 // The equations-of-motion residual at the forward substep's accelerations (see hostemu_residual).
 int spi_hostemu_residual(const spi_robot* robot, const double* state, const double* theta, const double* act12,

@@ -1,8 +1,14 @@
 // sensitivity.cu -- per-window state sensitivities d s_H / d theta and Fisher information.
 //
 // spi_sensitivity: forward-mode (tangent-linear) derivatives of every window's final state
-// with respect to K theta slots, for N theta samples: one lane quad per (sample, window,
-// direction), running the templated dynamics with the dual scalar Df (value + one tangent).
+// with respect to K theta slots, for N theta samples. Two ways:
+//   * every direction by the dual scalar Df (value + one tangent) through the templated dynamics,
+//     one lane quad per (sample, window, direction). Each direction carries the whole trajectory, the
+//     legs' condensation and the Cholesky factorisation along: some 4,000 instructions a substep;
+//   * the first direction that way, keeping each substep's solve, and the others by tangent.cuh from
+//     the kept substeps, one quad per (sample, window, direction) too, a quarter of the instructions.
+// The second runs two chains one after the other, so it takes over where the dual rollouts no longer
+// fit the GPU at once (use_tangents).
 // With K <= 13 parameters and a 37-dimensional state, K forward tangents give the whole
 // Jacobian J_w (37 x K) of each window -- cheaper than 37 reverse (adjoint) sweeps -- and the
 // cost gradient follows as dc/dtheta = (dc/ds_H) J_w without checkpointing.
@@ -13,11 +19,14 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "dual.cuh"
 #include "engine_impl.h"
+#include "kept.cuh"
 #include "rollout.cuh"
+#include "tangent.cuh"
 
 using namespace spi;
 
@@ -44,29 +53,64 @@ __device__ __forceinline__ void dq_sum_out(LegOut<Df>& o) {
 }
 
 struct SensArgs {
-  const int* param_ids;  // [K] device
-  int K;
-  int N;
+  int ids[SPI_THETA_DIM];   // the theta slot of each direction
+  int K;                 // directions: the columns of J
+  long long nw0, nw;     // this launch's (sample, window) pairs
   float* J;              // [N][W][37][K]
   float* xH;             // [N][W][37] or null
+  float4* legs;          // kept substeps of the launch's pairs (kept.cuh)
+  float4* base;
+
+  __device__ __forceinline__ Kept kept(long long r, int leg) const { return Kept::of(legs, base, (size_t)nw, (size_t)r, leg); }
 };
 
-// One lane quad per (sample n, window w, direction k); 8 quads per warp.
+// The work record of the dual rollout that keeps its substeps: also the inverse pivots and the
+// contact's branch.
+struct DualWork : LegWork<Df> {
+  float diag[3], zf, fn, scale;
+  __device__ __forceinline__ void put_diag(Df a, Df b, Df c) { diag[0] = a.v; diag[1] = b.v; diag[2] = c.v; }
+  __device__ __forceinline__ void put_contact(Df z, const Df* branch) { zf = z.v; fn = branch[0].v; scale = branch[1].v; }
+};
+__device__ __forceinline__ SV<float> values(const SV<Df>& a) {
+  SV<float> r;
+  r.w = v3(a.w.x.v, a.w.y.v, a.w.z.v);
+  r.v = v3(a.v.x.v, a.v.y.v, a.v.z.v);
+  return r;
+}
+__device__ __forceinline__ BaseState<float> values(const BaseState<Df>& B) {
+  BaseState<float> r;
+  r.p = v3(B.p.x.v, B.p.y.v, B.p.z.v);
+  r.qx = B.qx.v; r.qy = B.qy.v; r.qz = B.qz.v; r.qw = B.qw.v;
+  r.nu = values(B.nu);
+  return r;
+}
+__device__ __forceinline__ LegState<float> values(const LegState<Df>& L) {
+  LegState<float> r;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) { r.q[k] = L.q[k].v; r.qd[k] = L.qd[k].v; }
+  return r;
+}
+
+// KEEP = false: one lane quad per (pair, direction k < K), 8 quads per warp. KEEP = true: direction 0 only, one
+// quad per pair, keeping every substep and the final state.
+template <bool KEEP>
 __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __restrict__ model, WinView win,
-                                                          const float* __restrict__ theta, SensArgs a) {
+                                                          const float* __restrict__ theta,
+                                                          const __grid_constant__ SensArgs a) {
   __shared__ DevModel M;
   load_model_smem(&M, model);
   __syncthreads();
   const int lane = threadIdx.x & 31, leg = lane & 3;
-  const long long total = (long long)a.N * win.W * a.K;
+  const int per = KEEP ? 1 : a.K;
+  const long long total = a.nw * per;
   long long q = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   const bool active = q < total;
   if (!active) q = total - 1;
-  const int k = (int)(q % a.K);
-  const long long nw = q / a.K;
+  const int k = (int)(q % per);
+  const long long r = q / per, nw = a.nw0 + r;
   const int w = (int)(nw % win.W), n = (int)(nw / win.W);
   const int W = win.W, H = win.H;
-  const int slot = a.param_ids[k];
+  const int slot = a.ids[k];
 
   Df th[SPI_THETA_DIM];
 #pragma unroll
@@ -91,18 +135,53 @@ __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __rest
     const float* ap = win.act + ((size_t)h * W + w) * 12 + 3 * leg;
     Df act[3] = {Df(__ldg(ap)), Df(__ldg(ap + 1)), Df(__ldg(ap + 2))};
     for (int s = 0; s < M.decimation; ++s) {
-      LegWork<Df> lw;
-      LegOut<Df> o = phase_a(M, leg, B, L, lp, act, lw);
-      dq_sum_out(o);
-      SV<Df> a0 = phase_b(M, bp, o, B);
-      phase_c(M, leg, a0, lw, L);
+      if (KEEP) {
+        const Kept kept = a.kept(r, leg);
+        const int at = h * M.decimation + s;
+        keep_state(kept, at, leg, values(B));
+        const float nuz = B.nu.v.z.v;
+        DualWork lw;
+        LegOut<Df> o = phase_a(M, leg, B, L, lp, act, lw);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const SV<float> v = values(lw.Kp[c]);
+          const float l = c == 0 ? lw.l10.v : (c == 1 ? lw.l20.v : lw.l21.v);
+          __stcs(kept.leg_at(at, 2 * c), make_float4(v.w.x, v.w.y, v.w.z, v.v.x));
+          __stcs(kept.leg_at(at, 2 * c + 1), make_float4(v.v.y, v.v.z, lw.y[c].v, l));
+        }
+        keep_legs(kept, at, lw.diag, values(L), lw.zf, (lw.fn > 0.f ? 1.f : 0.f) + (lw.scale == M.ct ? 2.f : 0.f));
+        dq_sum_out(o);
+        Art<Df> IA = rigid(bp.m, bp.h, bp.Io);
+        add_to(IA, o.I);
+        const SV<Df> pA = crf_acc(B.nu, rigid_mul(bp.m, bp.h, bp.Io, B.nu), o.p);
+        V3<Df> d;
+        Factor6 fac;
+        const SV<Df> a0 = base_solve_step(M, IA, pA, B, d, fac);
+        B.p = B.p + d;
+        keep_solve(kept, at, leg, nuz, values(a0), fac);
+        phase_c(M, leg, a0, lw, L);
+      } else {
+        LegWork<Df> lw;
+        LegOut<Df> o = phase_a(M, leg, B, L, lp, act, lw);
+        dq_sum_out(o);
+        SV<Df> a0 = phase_b(M, bp, o, B);
+        phase_c(M, leg, a0, lw, L);
+      }
     }
+  }
+  if (KEEP) {
+    const Kept kept = a.kept(r, leg);
+    const int at = H * M.decimation;
+    const float none[3] = {0.f, 0.f, 0.f};
+    keep_state(kept, at, leg, values(B));
+    if (leg == 0) *kept.base_at(at, 3) = make_float4(B.nu.v.z.v, 0.f, 0.f, 0.f);
+    keep_legs(kept, at, none, values(L));
   }
   if (!active) return;
   Df s13[13];
   base_to_world(B, s13);
-  float* Jp = a.J + (((size_t)n * W + w) * SPI_STATE_DIM) * a.K + k;
-  float* xp = a.xH ? a.xH + ((size_t)n * W + w) * SPI_STATE_DIM : nullptr;
+  float* Jp = a.J + ((size_t)nw * SPI_STATE_DIM) * a.K + k;
+  float* xp = a.xH ? a.xH + (size_t)nw * SPI_STATE_DIM : nullptr;
   if (leg == 0) {
 #pragma unroll
     for (int i = 0; i < 13; ++i) {
@@ -119,6 +198,147 @@ __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __rest
       xp[25 + 3 * leg + j] = L.qd[j].v;
     }
   }
+}
+
+constexpr int kKeptFields = 4 * kLegFields + kBaseFields;   // a kept substep of one rollout
+
+// Directions 1 .. K - 1 from the kept substeps, one lane quad per (pair, direction), a pair's directions side by
+// side. The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
+// asynchronous copies two substeps ahead, three buffers in turn; read straight from memory, two warps per
+// scheduler waited for each substep's loads twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
+__global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict__ model, WinView win,
+                                                      const float* __restrict__ theta,
+                                                      const __grid_constant__ SensArgs a, int stage_pairs) {
+  extern __shared__ float4 stage[];               // [3][stage_pairs][kKeptFields]
+  __shared__ DevModel M;
+  load_model_smem(&M, model);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, leg = lane & 3;
+  const long long total = a.nw * (a.K - 1);
+  const long long q0 = (long long)blockIdx.x * 32;
+  long long q = q0 + (threadIdx.x >> 2);
+  const bool active = q < total;
+  if (!active) q = total - 1;
+  const long long first = q0 / (a.K - 1);
+  const int pairs = (int)(min(q0 + 31, total - 1) / (a.K - 1) - first) + 1;   // <= stage_pairs
+  const int k = 1 + (int)(q % (a.K - 1));
+  const long long r = q / (a.K - 1), nw = a.nw0 + r;
+  const int W = win.W, H = win.H, w = (int)(nw % W), n = (int)(nw / W);
+  const int slot = a.ids[k];
+  float th[SPI_THETA_DIM];
+#pragma unroll
+  for (int i = 0; i < SPI_THETA_DIM; ++i) th[i] = __ldg(theta + (size_t)n * SPI_THETA_DIM + i);
+  const BaseParams<float> bp = base_params<float>(M, th);
+  const LegParams<float> lp = leg_params<float>(th, leg);
+  tng::ParamTan<float> dP;
+  tng::base_params_tan(M, th, slot, dP.m, dP.h, dP.Io);
+  const int s0 = leg >= 2 ? 9 : 5;
+  dP.kps = slot == s0 ? 1.f : 0.f;
+  dP.fc = slot == s0 + 1 ? 1.f : 0.f;
+  dP.arm = slot == s0 + 2 ? 1.f : 0.f;
+  dP.ts = slot == s0 + 3 ? 1.f : 0.f;
+  const int last = H * M.decimation;               // the slot of the final state
+  auto fetch = [&](int at) {
+    if (at <= last)
+      for (int i = threadIdx.x; i < pairs * kKeptFields; i += blockDim.x) {
+        const int p = i / kKeptFields, f = i - p * kKeptFields;
+        const Kept from = a.kept(first + p, f < 4 * kLegFields ? f / kLegFields : 0);
+        const float4* src = f < 4 * kLegFields ? from.leg_at(at, f % kLegFields) : from.base_at(at, f - 4 * kLegFields);
+        copy_async(stage + ((at % 3) * stage_pairs + p) * kKeptFields + f, src);
+      }
+    copy_async_commit();
+  };
+  auto view = [&](int at) {
+    const float4* f = stage + ((at % 3) * stage_pairs + (int)(r - first)) * kKeptFields;
+    return KeptView{f + leg * kLegFields, f + 4 * kLegFields};
+  };
+  auto arrive = [&] {
+    copy_async_wait<0>();
+    __syncthreads();
+  };
+  fetch(0);
+  fetch(1);
+  arrive();
+  BaseState<float> B0 = view(0).state();
+  tng::BaseTan<float> dB = tng::zero_base_tan<float>();
+  tng::LegTan<float> dL = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+  for (int h = 0; h < H; ++h) {
+    float tgt[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      tgt[j] = joint_target(M, j, leg, __ldg(win.act + ((size_t)h * W + w) * 12 + 3 * leg + j));
+    for (int s = 0; s < M.decimation; ++s) {
+      const int at = h * M.decimation + s;
+      if (at > 0) arrive();                        // slot at + 1 is here, slot at - 1 is free
+      fetch(at + 2);
+      const KeptView now = view(at);
+      const LegState<float> L = now.leg_state();
+      const float4 c = now.legf(8);
+      const int branch = (int)c.z;
+      const tng::ContactBranch br = {(branch & 1) != 0, (branch & 2) != 0};
+      const SV<float> a0 = now.accel();
+      float qdd[3], dr[3], z[3], dqdd[3];
+      SV<float> x;
+      {
+        float res[3];
+        SV<float> fb;
+        adj::leg_qdd(now.work(), a0, qdd);
+        adj::LegTape<float> t;
+        adj::leg_pose(B0, L, t);
+        adj::leg_residual<kMotorRuntime>(M, leg, B0, L, lp, tgt, a0, qdd, t, res, fb);
+        tng::leg_residual_tan(M, leg, B0, L, lp, tgt, qdd, t, c.y, br, dB, dL, dP, dr, x);
+      }
+      if (corners_may_touch(M, B0)) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          adj::add_sv(x, tng::corner_residual_tan(M, B0, lc_corner<float>(M.legc[leg], j), a0, dB));
+      }
+      // M' da = -dr
+      const float lam[3] = {-dr[0], -dr[1], -dr[2]};
+      const adj::SolveWork<float> sw = now.work();
+      adj::add_sv(x, adj::leg_solve_down(sw, lam, z));
+      qsum3(x.w);
+      qsum3(x.v);
+      adj::add_sv(x, tng::base_residual_tan(bp, B0, a0, dB, dP));
+      const SV<float> da0 = now.factor().solve(adj::sub_sv(adj::zsv<float>(), x));
+      adj::leg_solve_up(sw, z, da0, dqdd);
+      const BaseState<float> B1 = view(at + 1).state();
+      tng::base_integrate_tan(M, B0, B1, da0, dB);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        dL.qd[j] = dL.qd[j] + M.dt * dqdd[j];
+        dL.q[j] = dL.q[j] + M.dt * dL.qd[j];
+      }
+      B0 = B1;
+    }
+  }
+  if (!active) return;
+  float s13[13];
+  tng::base_to_world_tan(B0, dB, s13);
+  float* Jp = a.J + ((size_t)nw * SPI_STATE_DIM) * a.K + k;
+  if (leg == 0) {
+#pragma unroll
+    for (int i = 0; i < 13; ++i) Jp[(size_t)i * a.K] = s13[i];
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    Jp[(size_t)(13 + 3 * leg + j) * a.K] = dL.q[j];
+    Jp[(size_t)(25 + 3 * leg + j) * a.K] = dL.qd[j];
+  }
+}
+
+constexpr size_t kScratch = (size_t)4 << 30;   // bytes of kept substeps
+
+// Whether the directions past the first go by tangents: three directions or more whose dual rollouts would
+// take more than `waves` times the warps that fit the GPU at once (two CTAs of 255 registers a thread per
+// SM). The first direction's chain comes before the others', so below two waves the dual rollouts are done
+// first, and with two directions it does not come back (H = 20, 152 SMs, dual against tangents):
+//   1100 pairs x 13   0.77 / 0.92 ms      1530 x 13   1.13 / 0.93 ms      4096 x 13   2.30 / 1.69 ms
+//   4900 pairs x 3    0.79 / 0.95 ms      6600 x 3    1.13 / 1.03 ms     10000 x 2    1.13 / 1.35 ms
+// Batches follow one another, each with a last wave of its own; several of them need twice as much each.
+constexpr int kDualWaves = 2;
+bool use_tangents(long long pairs, int K, int sms, int waves) {
+  return K >= 3 && pairs * K > (long long)waves * 2 * 32 * sms;
 }
 
 // ---------------------------------------------------------------------------
@@ -292,16 +512,44 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
   for (int k = 0; k < K; ++k)
     if (param_ids[k] < 0 || param_ids[k] >= SPI_THETA_DIM)
       return set_error(SPI_EINVAL, "spi_sensitivity: param_ids[%d]=%d", k, param_ids[k]);
-  int rc = e->sens_ids.reserve(SPI_THETA_DIM * sizeof(int));
-  if (rc) return rc;
-  memcpy(e->h_sens_ids, param_ids, K * sizeof(int));
-  cudaError_t ce = cudaMemcpyAsync(e->sens_ids.p, e->h_sens_ids, K * sizeof(int), cudaMemcpyHostToDevice, e->stream);
-  if (ce != cudaSuccess) return cuda_error(ce, "spi_sensitivity: ids");
-  WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
-  SensArgs a{(const int*)e->sens_ids.p, K, N, J, xH};
-  const long long quads = (long long)N * e->W * K;
-  sensitivity_kernel<<<(unsigned)((quads + 31) / 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
-  ce = cudaGetLastError();
+  const WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
+  SensArgs a{};
+  for (int k = 0; k < K; ++k) a.ids[k] = param_ids[k];
+  a.K = K;
+  a.J = J;
+  a.xH = xH;
+  const long long all = (long long)N * e->W;
+  const size_t slots = (size_t)e->H * e->host_model.decimation + 1;
+  // batches of equal size within kScratch. A capture keeps to the dual rollouts, which need no memory of the
+  // engine's: a graph would go on using what a later call may replace.
+  const long long most = std::max(1LL, (long long)(kScratch / (slots * kKeptBytes)));
+  const long long batches = (all + most - 1) / most;
+  long long batch = (all + batches - 1) / batches;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool split = use_tangents(batch, K, e->sms, batches > 1 ? 2 * kDualWaves : kDualWaves) &&
+                     cudaStreamIsCapturing(e->stream, &capture) == cudaSuccess &&
+                     capture == cudaStreamCaptureStatusNone &&
+                     e->sens_kept.reserve(slots * batch * kKeptBytes) == SPI_OK;
+  if (!split) batch = all;
+  const int stage_pairs = split ? 31 / (K - 1) + 2 : 0;   // pairs that 32 consecutive quads can touch, at most
+  const int smem = 3 * stage_pairs * kKeptFields * (int)sizeof(float4);
+  if (split) {
+    const cudaError_t fe = cudaFuncSetAttribute(tangent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (fe != cudaSuccess) return cuda_error(fe, "spi_sensitivity: shared memory");
+  }
+  for (long long r0 = 0; r0 < all; r0 += batch) {
+    a.nw0 = r0;
+    a.nw = std::min(batch, all - r0);
+    if (split) {
+      a.legs = (float4*)e->sens_kept.p;
+      a.base = a.legs + slots * kLegFields * 4 * a.nw;
+      sensitivity_kernel<true><<<blocks_for(a.nw, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
+      tangent_kernel<<<blocks_for(a.nw * (K - 1), 32), 128, smem, e->stream>>>(e->d_model, win, theta, a, stage_pairs);
+    } else {
+      sensitivity_kernel<false><<<blocks_for(a.nw * K, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
+    }
+  }
+  const cudaError_t ce = cudaGetLastError();
   return ce == cudaSuccess ? SPI_OK : cuda_error(ce, "spi_sensitivity: launch");
 }
 

@@ -112,6 +112,9 @@ def hostemu_lib():
         lib.spi_hostemu_grad.restype = c_int
         lib.spi_hostemu_grad.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                          c_int, c_int, c_void_p, c_void_p]
+        lib.spi_hostemu_tangent.restype = c_int
+        lib.spi_hostemu_tangent.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                                            c_void_p]
         lib.spi_hostemu_residual.restype = c_int
         lib.spi_hostemu_residual.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p, c_void_p]
         _hostemu = lib

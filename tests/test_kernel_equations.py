@@ -143,6 +143,33 @@ def test_hip_frame_legs_equal_articulated_body_algorithm(built, kw):
     assert np.abs(out[0] - out[1]).max() < 1e-9
 
 
+@pytest.mark.parametrize("kw", [dict(), dict(torque_speed=False, inertia_follows_mass=True),
+                                dict(tanh_a=(15.0, 18.0, 25.0), motor_gain=(0.9, 1.1, 1.05))])
+def test_substep_tangents_equal_central_differences(built, kw):
+    """The substep tangents (csrc/tangent.cuh) in FP64 against central differences of the rollout (h = 1e-6:
+    truncation and rounding each some 1e-9 of entries up to 1e2, hence 1e-4 with room for the curvature of
+    contacts): feet in and out of contact, a base on the ground, saturated motors."""
+    from spi_gb300 import _lib, robot
+    _, x0, acts, th = _inputs(21, B=6, H=8)
+    x0[3:5, 2] = 0.26
+    x0[5, 2] = 0.06
+    acts[4] *= 30
+    r, lib = robot.to_struct(robot.SimConfig(**kw)), _lib.hostemu_lib()
+    x0, acts, th = (np.ascontiguousarray(a, dtype=np.float64) for a in (x0, acts, th))
+    for b in range(6):
+        for k in range(13):
+            state, d, ends = np.zeros(37), np.zeros(37), np.zeros((2, 8, 37))
+            assert lib.spi_hostemu_tangent(ctypes.byref(r), x0[b].ctypes.data, acts[b].ctypes.data, th[b].ctypes.data, k, 8,
+                                           state.ctypes.data, d.ctypes.data) == 0
+            two = np.stack([th[b], th[b]])
+            two[:, k] += (1e-6, -1e-6)
+            x, a = np.stack([x0[b]] * 2), np.stack([acts[b]] * 2)
+            assert lib.spi_hostemu_rollout(ctypes.byref(r), x.ctypes.data, a.ctypes.data, two.ctypes.data, 2, 8,
+                                           ends.ctypes.data) == 0
+            ref = (ends[0, -1] - ends[1, -1]) / 2e-6
+            assert np.linalg.norm(d - ref) <= 1e-4 * max(np.linalg.norm(ref), 1e-2), (b, k)
+
+
 def test_kernel_vs_oracle_with_urdf_constants(built):
     """Float32 model constants move states by < 1e-5 (well inside the 1e-4 parity bar)."""
     cfg, x0, acts, th = _inputs(13)
