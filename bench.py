@@ -348,13 +348,14 @@ def run_c3(args):
     from spi_gb300.engine import probe_fp32_peak
     from spi_gb300.flops import dual_flops_per_rollout_step
     dual_fl = dual_flops_per_rollout_step(cfg)
-    sens_roof = {"kernel": "sensitivity_kernel", "bound": "fp32",
+    sens_roof = {"kernel": "sensitivity_kernel, tangent_kernel", "bound": "fp32",
                  "achieved": n * wpc * H * 13 * dual_fl / (breakdown["sensitivities_ms"] * 1e-3) / 1e12,
                  "peak": probe_fp32_peak() / 1e12, "unit": "TFLOP/s",
                  "flops_per_tangent_rollout_step": dual_fl,
                  "note": "achieved = tangent rollout-steps x FP operations of one dual-number control step "
                          "(csrc/dual.cuh arithmetic, counted on the host; phase B once) / the sensitivity "
-                         "phase's device time; peak: the FP32 FMA-loop probe of this GPU"}
+                         "phase's device time; the directions past the first take fewer operations "
+                         "(csrc/tangent.cuh), so this is the rate of the dual-number work replaced; peak: the FP32 FMA-loop probe of this GPU"}
     sens_roof["frac"] = sens_roof["achieved"] / sens_roof["peak"]
     # the Fisher reduction alone, tensor cores against CUDA cores, on the last Jacobians
     J, q = r["J"], block_weights((10.0, 5.0, 0.1, 0.1, 1.0, 0.01))
@@ -376,11 +377,11 @@ def run_c3(args):
     f_s = fisher_ms["tensor_cores_bf16"] * 1e-3
     bf16_peak = peaks.get("bf16_tflops", 1900.0)
     hbm_peak = peaks.get("hbm_gbs", 6800.0)
-    fisher_roof = {"kernel": "fisher_mma_kernel", "bound": "hbm", "achieved": f_bytes / f_s / 1e9, "peak": hbm_peak,
+    fisher_roof = {"kernel": "fisher_kernel<true>", "bound": "hbm", "achieved": f_bytes / f_s / 1e9, "peak": hbm_peak,
                    "unit": "GB/s", "frac": f_bytes / f_s / 1e9 / hbm_peak,
                    "tensor_tflops": f_flops / f_s / 1e12, "tensor_frac": f_flops / f_s / 1e12 / bf16_peak,
                    "note": "13 x 13 Gram matrices over 296 rows per candidate: too small for either roof "
-                           "(one warp per candidate, latency-bound); peaks from MEASURED_PEAKS.json"}
+                           "(one CTA per two candidates, latency-bound); peaks from MEASURED_PEAKS.json"}
     fd_line = fd_fisher_throughput(eng, acts, args)
     grad_line = gradient_throughput(eng, args)
     tangent_steps = n * wpc * H * 13
@@ -535,8 +536,7 @@ def fd_fisher_throughput(eng, acts, args, param_ids=tuple(range(13)), delta=0.1,
 def gradient_throughput(eng, args, n_theta=512, n_windows=256, horizon=20):
     """d cost / d theta of the squared-error window cost for n_theta prior samples against
     n_windows windows x H = 20 (13 parameters): one hand-written adjoint sweep per rollout
-    (spi_adjoint, checkpoints every 5 control steps) against 13 forward-mode tangent sweeps
-    (spi_sensitivity). CUDA-event times on the engine stream after a warm-up call of each."""
+    (spi_adjoint) against 13 forward-mode directions (spi_sensitivity). CUDA-event times on the engine stream after a warm-up call of each."""
     import torch
     from spi_gb300 import robot
     from spi_gb300.data import synthetic_windows

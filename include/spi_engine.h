@@ -200,7 +200,9 @@ int spi_cem_read(spi_engine* e, double* mu, double* cov, float* best_theta, floa
  * trace(J^T J)) with exact forward-mode derivatives of the rollout.
  * spi_sensitivity: J[n][w][i][k] = d s_H[i] / d theta[param_ids[k]] of window w (the loaded
  * windows) for theta sample n (device [N][13]); J device [N][W][37][K]; xH device
- * [N][W][37] final states or NULL. K <= 13. Asynchronous on the engine stream.
+ * [N][W][37] final states or NULL. K <= 13. Three directions or more of many pairs keep the first
+ * direction's substeps in engine memory (4 GB at most; without it, and in a stream capture, every
+ * direction runs its own rollout). Asynchronous on the engine stream.
  * spi_fisher: F[n] = sum_w J_w^T diag(state_weight) J_w (device [N][K][K], FP32
  * accumulation), logdet[n] = log det(F[n] + eps I) and trace[n] = trace(F[n]) in FP64
  * (device [N] each, may be NULL). */
@@ -219,8 +221,10 @@ int spi_fisher_ex(const float* J, int N, int W, int K, const float* state_weight
  * theta device [N][13] against the loaded windows, cost[n] = the engine's cost (spi_set_cost
  * mode and weights, the window weights and normaliser of spi_load_windows) and grad[n][13] =
  * d cost[n] / d theta[n] by a hand-written reverse sweep of the rollout: the forward pass keeps
- * the state every 5 control steps, the reverse pass recomputes each 5-step segment forward and
- * runs the substep adjoints backwards through it. cost and grad are device pointers (either may
+ * what each physics substep was solved with (736 bytes a rollout), the reverse pass runs the
+ * substep adjoints backwards from it. The kept substeps take 4 GB of engine memory at most:
+ * (theta, 8-window group) pairs go through in batches (smaller ones if the device has less to
+ * give), horizons over 50 control steps in segments. cost and grad are device pointers (either may
  * be NULL). Non-finite final states are counted as by spi_run (spi_sync). Asynchronous on the
  * engine stream. */
 int spi_adjoint(spi_engine* e, const float* theta, int N, float* cost, float* grad);
@@ -266,7 +270,7 @@ int spi_fd_fisher(spi_engine* e, const float* x0, const float* actions, const fl
  * 8-window group), one warp each, laid out longest horizon first), and finished jobs free
  * their slot and memory for the next arrivals. One tick is captured once as a CUDA graph. A
  * job's results do not depend on the other jobs in the mix, and equal the single-job engine's
- * (spi_cem_*) bit for bit: the server and spi_run launch the same compiled rollout kernel.
+ * (spi_cem_*) bit for bit: the server and the engine CEM launch the same compiled rollout kernel.
  * No counterpart in the reference, which runs one job at a time. */
 typedef struct spi_server spi_server;
 

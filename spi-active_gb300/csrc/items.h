@@ -1,9 +1,10 @@
-// items.h -- the rollout kernels of the single-job engine and of the server, one compiled copy each.
+// items.h -- the rollout kernels of the engine CEM and of the server, one compiled copy each.
 //
-// Both the engine (spi_run, the engine CEM) and the continuous-batching server (spi_server_tick)
-// evaluate their (theta, window) pairs with the same kernels, defined once in items.cu: every
-// warp takes a work item and looks up, in a slot table, which job the item belongs to. The
-// engine is a table of one slot. Because both callers launch
+// Both the engine CEM (and spi_run in the quad layout) and the continuous-batching server
+// (spi_server_tick) evaluate their (theta, window) pairs with the same kernels, defined once in
+// items.cu: every warp takes a work item and looks up, in a slot table, which job the item belongs
+// to. The engine is a table of one slot. (spi_run in the lane layout on a population that the CEM did
+// not draw, and spi_evaluate, take the kernels of eval.cu.) Because both callers launch
 // the same compiled kernel, a job's costs are bitwise identical whether it runs alone on the
 // engine or inside the server's mix; two separately compiled copies of the rollout may contract
 // different multiply-add pairs into FMAs and differ in the last bit.

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __rest
 constexpr int kKeptFields = 4 * kLegFields + kBaseFields;   // a kept substep of one rollout
 
 // Directions 1 .. K - 1 from the kept substeps, one lane quad per (pair, direction), a pair's directions side by
-// side. The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
+// side. Bound by its arithmetic at the 8 warps per SM that 255 registers leave (0.67 instructions a cycle). The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
 // asynchronous copies two substeps ahead, three buffers in turn; read straight from memory, two warps per
 // scheduler waited for each substep's loads twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
 __global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict__ model, WinView win,

@@ -4,7 +4,7 @@
 // A tick advances every active slot by one CEM iteration:
 //   cem_sample_kernel (grid row per slot) -> the rollout kernel of items.cu (one warp per
 //   (slot, theta, 8-window group) work item, items ordered longest horizon first; the
-//   single-job engine launches the same kernel on a one-slot table) -> server_finalize_kernel
+//   engine CEM launches the same kernel on a one-slot table) -> server_finalize_kernel
 //   -> cem_refit_kernel.
 // The tick is captured once as a CUDA graph: every per-tick quantity (slot table, work
 // order, item count) lives in device buffers that the host refreshes before each launch, and

@@ -60,7 +60,7 @@ def block_weights(sq_weights):
 
 def adjoint(engine, theta):
     """(cost [N], d cost / d theta [N, 13]) of the engine's cost by the hand-written adjoint
-    (spi_adjoint): one reverse sweep per rollout, checkpoints every 5 control steps."""
+    (spi_adjoint): one reverse sweep per rollout, from substeps that its forward pass keeps."""
     theta = torch.as_tensor(theta, dtype=torch.float32, device=engine.device).reshape(-1, THETA_DIM).contiguous()
     N = theta.shape[0]
     cost = torch.empty((N,), device=engine.device)
