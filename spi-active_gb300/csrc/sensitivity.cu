@@ -201,15 +201,58 @@ __global__ void __launch_bounds__(128) sensitivity_kernel(const DevModel* __rest
 }
 
 constexpr int kKeptFields = 4 * kLegFields + kBaseFields;   // a kept substep of one rollout
+constexpr int kTapeFields = 25;   // a leg's tape (24, and one that sets the legs four banks apart)
+
+// What leg_residual_tan reads of a leg's tape, and the joint accelerations.
+__device__ __forceinline__ void store_tape(float4* d, const adj::LegTape<float>& t, const float qdd[3]) {
+  d[0] = make_float4(t.c[0], t.c[1], t.c[2], t.mimp);
+  d[1] = make_float4(t.s[0], t.s[1], t.s[2], t.vf.x);
+  d[2] = make_float4(t.vf.y, t.vf.z, qdd[0], qdd[1]);
+  const SV<float> v[12] = {t.v0, t.v1, t.v2, t.al0, t.al1, t.al2, t.h0, t.h1, t.h2, t.f0, t.f1, t.f2};
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    const SV<float>&a = v[2 * i], &b = v[2 * i + 1];
+    d[3 + 3 * i] = make_float4(a.w.x, a.w.y, a.w.z, a.v.x);
+    d[4 + 3 * i] = make_float4(a.v.y, a.v.z, b.w.x, b.w.y);
+    d[5 + 3 * i] = make_float4(b.w.z, b.v.x, b.v.y, b.v.z);
+  }
+  d[21] = make_float4(t.g1.x, t.g1.y, t.g1.z, t.g2.x);
+  d[22] = make_float4(t.g2.y, t.g2.z, t.g3.x, t.g3.y);
+  d[23] = make_float4(t.g3.z, qdd[2], 0.f, 0.f);
+}
+__device__ __forceinline__ void load_tape(const float4* d, adj::LegTape<float>& t, float qdd[3]) {
+  t.c[0] = d[0].x; t.c[1] = d[0].y; t.c[2] = d[0].z; t.mimp = d[0].w;
+  t.s[0] = d[1].x; t.s[1] = d[1].y; t.s[2] = d[1].z;
+  t.vf = v3(d[1].w, d[2].x, d[2].y);
+  qdd[0] = d[2].z; qdd[1] = d[2].w; qdd[2] = d[23].y;
+  SV<float>* const v[12] = {&t.v0, &t.v1, &t.v2, &t.al0, &t.al1, &t.al2, &t.h0, &t.h1, &t.h2, &t.f0, &t.f1, &t.f2};
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    SV<float>&a = *v[2 * i], &b = *v[2 * i + 1];
+    const float4 x = d[3 + 3 * i], y = d[4 + 3 * i], z = d[5 + 3 * i];
+    a.w = v3(x.x, x.y, x.z); a.v = v3(x.w, y.x, y.y);
+    b.w = v3(y.z, y.w, z.x); b.v = v3(z.y, z.z, z.w);
+  }
+  t.g1 = v3(d[21].x, d[21].y, d[21].z);
+  t.g2 = v3(d[21].w, d[22].x, d[22].y);
+  t.g3 = v3(d[22].z, d[22].w, d[23].x);
+}
 
 // Directions 1 .. K - 1 from the kept substeps, one lane quad per (pair, direction), a pair's directions side by
 // side. Bound by its arithmetic at the 8 warps per SM that 255 registers leave (0.67 instructions a cycle). The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
 // asynchronous copies two substeps ahead, three buffers in turn; read straight from memory, two warps per
 // scheduler waited for each substep's loads twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
-__global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict__ model, WinView win,
+//
+// TAPES: the part of the residual that a pair's directions share (sines, velocities, accelerations, forces: a
+// third of a direction's instructions) is formed once per pair, a substep ahead, one lane per leg, the
+// warps taking turns, and read from shared memory. Without its registers three CTAs fit an SM. The
+// results are the same to the bit.
+template <bool TAPES>
+__global__ void __launch_bounds__(128, TAPES ? 3 : 2) tangent_kernel(const DevModel* __restrict__ model, WinView win,
                                                       const float* __restrict__ theta,
                                                       const __grid_constant__ SensArgs a, int stage_pairs) {
   extern __shared__ float4 stage[];               // [3][stage_pairs][kKeptFields]
+  float4* const tapes = stage + 3 * stage_pairs * kKeptFields;   // [2][stage_pairs][4][kTapeFields]
   __shared__ DevModel M;
   load_model_smem(&M, model);
   __syncthreads();
@@ -248,9 +291,28 @@ __global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict
       }
     copy_async_commit();
   };
-  auto view = [&](int at) {
-    const float4* f = stage + ((at % 3) * stage_pairs + (int)(r - first)) * kKeptFields;
+  auto view_of = [&](int at, int p) {
+    const float4* f = stage + ((at % 3) * stage_pairs + p) * kKeptFields;
     return KeptView{f + leg * kLegFields, f + 4 * kLegFields};
+  };
+  auto tape = [&](int at, int p) { return tapes + (((at & 1) * stage_pairs + p) * 4 + leg) * kTapeFields; };
+  auto view = [&](int at) { return view_of(at, (int)(r - first)); };
+  const int warp = threadIdx.x >> 5;
+  // the CTA's tapes of a substep, one lane per leg of a pair, eight pairs a warp; the warps take turns
+  auto make_tapes = [&](int at) {
+    const int p = ((warp - at) & 3) * 8 + (lane >> 2);
+    if (p >= pairs) return;
+    const KeptView k = view_of(at, p);
+    const BaseState<float> B = k.state();
+    const LegState<float> L = k.leg_state();
+    const SV<float> a0 = k.accel();
+    float qdd[3], none[3] = {0.f, 0.f, 0.f}, res[3];   // (the torques do not enter the tape)
+    SV<float> fb;
+    adj::LegTape<float> t;
+    adj::leg_qdd(k.work(), a0, qdd);
+    adj::leg_pose(B, L, t);
+    adj::leg_residual<kMotorRuntime>(M, leg, B, L, lp, none, a0, qdd, t, res, fb);
+    store_tape(tape(at, p), t, qdd);
   };
   auto arrive = [&] {
     copy_async_wait<0>();
@@ -259,6 +321,10 @@ __global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict
   fetch(0);
   fetch(1);
   arrive();
+  if (TAPES) {
+    make_tapes(0);
+    __syncthreads();
+  }
   BaseState<float> B0 = view(0).state();
   tng::BaseTan<float> dB = tng::zero_base_tan<float>();
   tng::LegTan<float> dL = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
@@ -269,8 +335,9 @@ __global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict
       tgt[j] = joint_target(M, j, leg, __ldg(win.act + ((size_t)h * W + w) * 12 + 3 * leg + j));
     for (int s = 0; s < M.decimation; ++s) {
       const int at = h * M.decimation + s;
-      if (at > 0) arrive();                        // slot at + 1 is here, slot at - 1 is free
+      if (at > 0) arrive();                        // slot at + 1 and tape at are here, at - 1's are free
       fetch(at + 2);
+      if (TAPES && at + 1 < last) make_tapes(at + 1);
       const KeptView now = view(at);
       const LegState<float> L = now.leg_state();
       const float4 c = now.legf(8);
@@ -280,12 +347,16 @@ __global__ void __launch_bounds__(128) tangent_kernel(const DevModel* __restrict
       float qdd[3], dr[3], z[3], dqdd[3];
       SV<float> x;
       {
-        float res[3];
-        SV<float> fb;
-        adj::leg_qdd(now.work(), a0, qdd);
         adj::LegTape<float> t;
-        adj::leg_pose(B0, L, t);
-        adj::leg_residual<kMotorRuntime>(M, leg, B0, L, lp, tgt, a0, qdd, t, res, fb);
+        if (TAPES) {
+          load_tape(tape(at, (int)(r - first)), t, qdd);
+        } else {
+          float res[3];
+          SV<float> fb;
+          adj::leg_qdd(now.work(), a0, qdd);
+          adj::leg_pose(B0, L, t);
+          adj::leg_residual<kMotorRuntime>(M, leg, B0, L, lp, tgt, a0, qdd, t, res, fb);
+        }
         tng::leg_residual_tan(M, leg, B0, L, lp, tgt, qdd, t, c.y, br, dB, dL, dP, dr, x);
       }
       if (corners_may_touch(M, B0)) {
@@ -339,6 +410,14 @@ constexpr size_t kScratch = (size_t)4 << 30;   // bytes of kept substeps
 constexpr int kDualWaves = 2;
 bool use_tangents(long long pairs, int K, int sms, int waves) {
   return K >= 3 && pairs * K > (long long)waves * 2 * 32 * sms;
+}
+
+// Whether the tangents of a pair share one tape: with four or more to share it, and over two waves of the two
+// CTAs per SM that fit otherwise (H = 20, 152 SMs, whole call, own tapes against shared ones):
+//   4096 pairs x 13   1.69 / 1.55 ms      1650 x 13   1.06 / 1.00 ms      1530 x 13   0.86 / 0.92 ms
+//   8192 pairs x 5    1.43 / 1.40 ms      8192 x 4    1.25 / 1.34 ms
+bool use_tapes(long long pairs, int K, int sms) {
+  return K >= 5 && pairs * (K - 1) > (long long)2 * 2 * 32 * sms;
 }
 
 // ---------------------------------------------------------------------------
@@ -532,9 +611,11 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
                      e->sens_kept.reserve(slots * batch * kKeptBytes) == SPI_OK;
   if (!split) batch = all;
   const int stage_pairs = split ? 31 / (K - 1) + 2 : 0;   // pairs that 32 consecutive quads can touch, at most
-  const int smem = 3 * stage_pairs * kKeptFields * (int)sizeof(float4);
+  const bool tapes = use_tapes(batch, K, e->sms);
+  const int smem = stage_pairs * (3 * kKeptFields + (tapes ? 8 * kTapeFields : 0)) * (int)sizeof(float4);
+  const auto tangents = tapes ? tangent_kernel<true> : tangent_kernel<false>;
   if (split) {
-    const cudaError_t fe = cudaFuncSetAttribute(tangent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t fe = cudaFuncSetAttribute(tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (fe != cudaSuccess) return cuda_error(fe, "spi_sensitivity: shared memory");
   }
   for (long long r0 = 0; r0 < all; r0 += batch) {
@@ -544,7 +625,7 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
       a.legs = (float4*)e->sens_kept.p;
       a.base = a.legs + slots * kLegFields * 4 * a.nw;
       sensitivity_kernel<true><<<blocks_for(a.nw, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
-      tangent_kernel<<<blocks_for(a.nw * (K - 1), 32), 128, smem, e->stream>>>(e->d_model, win, theta, a, stage_pairs);
+      tangents<<<blocks_for(a.nw * (K - 1), 32), 128, smem, e->stream>>>(e->d_model, win, theta, a, stage_pairs);
     } else {
       sensitivity_kernel<false><<<blocks_for(a.nw * K, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
     }

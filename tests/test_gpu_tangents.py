@@ -10,9 +10,11 @@ pytestmark = pytest.mark.gpu
 
 
 # 257 windows a theta; three to thirteen directions, counts that do and do not divide a CTA's 32
-# quads; the first line's pairs are more than 4 GB of kept substeps hold
+# quads; the first line's pairs are more than 4 GB of kept substeps hold, the last three's share
+# their tapes
 @pytest.mark.parametrize("N,ids", [(281, (0, 11, 5)), (16, (0, 3, 7, 8, 12)), (10, (1, 2, 4, 5, 6, 9, 10, 12)),
-                                   (6, tuple(range(13)))])
+                                   (6, tuple(range(13))), (20, (0, 3, 7, 8, 12)), (12, (1, 2, 4, 5, 6, 9, 10, 12)),
+                                   (8, tuple(range(13)))])
 def test_tangents_agree_with_dual_rollouts(built, N, ids):
     """Final states to the bit, J within the 1e-3 that it is held to everywhere; a second call to the bit."""
     from spi_gb300.engine import Engine
