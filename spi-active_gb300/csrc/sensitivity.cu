@@ -239,7 +239,8 @@ __device__ __forceinline__ void load_tape(const float4* d, adj::LegTape<float>& 
 }
 
 // Directions 1 .. K - 1 from the kept substeps, one lane quad per (pair, direction), a pair's directions side by
-// side. Bound by its arithmetic at the 8 warps per SM that 255 registers leave (0.67 instructions a cycle). The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
+// side. Bound by its arithmetic at the 8 or 12 warps per SM that its registers leave (0.67, 0.63 instructions a
+// cycle; with TAPES the warps wait for the one that forms the next tape). The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
 // asynchronous copies two substeps ahead, three buffers in turn; read straight from memory, two warps per
 // scheduler waited for each substep's loads twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
 //
@@ -404,7 +405,7 @@ constexpr size_t kScratch = (size_t)4 << 30;   // bytes of kept substeps
 // take more than `waves` times the warps that fit the GPU at once (two CTAs of 255 registers a thread per
 // SM). The first direction's chain comes before the others', so below two waves the dual rollouts are done
 // first, and with two directions it does not come back (H = 20, 152 SMs, dual against tangents):
-//   1100 pairs x 13   0.77 / 0.92 ms      1530 x 13   1.13 / 0.93 ms      4096 x 13   2.30 / 1.69 ms
+//   1100 pairs x 13   0.77 / 0.92 ms      1530 x 13   1.13 / 0.93 ms      4096 x 13   2.30 / 1.55 ms
 //   4900 pairs x 3    0.79 / 0.95 ms      6600 x 3    1.13 / 1.03 ms     10000 x 2    1.13 / 1.35 ms
 // Batches follow one another, each with a last wave of its own; several of them need twice as much each.
 constexpr int kDualWaves = 2;
