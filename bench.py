@@ -461,14 +461,16 @@ def identification_report(cem, eng, theta_true):
 
 def run_rollout_case(args):
     """One rollout-kernel case for profilers: ground-truth windows generated on the GPU (one
-    trace-kernel launch), prior theta samples, `--runs` launches of spi_run with the chosen
-    variant, the last one timed with CUDA events. Under ncu, skip the first runs - 1 launches of
+    trace-kernel launch), a CEM population drawn from the prior (spi_run on one takes the kernel
+    that a CEM iteration does), `--runs` launches of spi_run with the chosen variant, the last one
+    timed with CUDA events. Under ncu, skip the first runs - 1 launches of
     the kernel with -s and capture one with -c 1."""
     import torch
     import __graft_entry__
     __graft_entry__.build()
     from spi_gb300 import robot
     from spi_gb300.autotune import set_variant
+    from spi_gb300.cem import CEM
     from spi_gb300.data import synthetic_windows
     from spi_gb300.engine import Engine
     torch.cuda.set_device(0)
@@ -477,7 +479,8 @@ def run_rollout_case(args):
     e = Engine()
     init, act, tgt = synthetic_windows(e, lo + (hi - lo) * rng.random(13), args.n_windows, args.horizon, seed=77)
     e.load_windows(torch.from_numpy(init), torch.from_numpy(act), torch.from_numpy(tgt))
-    e.set_theta(torch.from_numpy((lo + (hi - lo) * rng.random((args.n_theta, 13))).astype(np.float32)))
+    CEM(e, n_samples=args.n_theta, param_ids=list(range(13)), lo=lo, hi=hi, nominal=robot.THETA_NOMINAL,
+        elite_frac=C1["elite_frac"], seed=5).sample()
     set_variant(e, args.variant)
     for _ in range(args.runs - 1):
         e.run()
