@@ -546,6 +546,38 @@ int spi_hostemu_tangent(const spi_robot* robot, const double* init, const double
     }
   return SPI_OK;
 }
+// contact_tan (tangent.cuh) of a foot in FP32: z, v, n and the branch, along dz, dv, dn -> out = dF [3], d mimp.
+int spi_hostemu_contact_tan(const spi_robot* robot, float z, const float* v, const float* n, int on, int stick, float dz,
+                            const float* dv, const float* dn, float* out) {
+  DevModel M;
+  const char* why = "";
+  int rc = build_dev_model(*robot, &M, &why);
+  if (rc) return rc;
+  const tng::ContactBranch br = {on != 0, stick != 0};
+  const V3<float> dF = tng::contact_tan(M, M.foot_r, z, v3(v[0], v[1], v[2]), v3(n[0], n[1], n[2]), br, dz,
+                                        v3(dv[0], dv[1], dv[2]), v3(dn[0], dn[1], dn[2]), out[3]);
+  out[0] = dF.x; out[1] = dF.y; out[2] = dF.z;
+  return SPI_OK;
+}
+// corner_residual_tan (tangent.cuh) of one base-box corner (leg, j) in FP32: a level base at height z moving with
+// v [3], no acceleration, along a change dv [3] of its velocity -> out [6] = (moment, force).
+int spi_hostemu_corner_tan(const spi_robot* robot, int leg, int j, float z, const float* v, const float* dv, float* out) {
+  DevModel M;
+  const char* why = "";
+  int rc = build_dev_model(*robot, &M, &why);
+  if (rc) return rc;
+  BaseState<float> B = {};
+  B.p.z = z;
+  B.qw = 1.f;
+  B.R = quat_to_R(0.f, 0.f, 0.f, 1.f);
+  B.nu.v = v3(v[0], v[1], v[2]);
+  tng::BaseTan<float> dB = tng::zero_base_tan<float>();
+  dB.nu.v = v3(dv[0], dv[1], dv[2]);
+  const SV<float> o = tng::corner_residual_tan(M, B, lc_corner<float>(M.legc[leg], j), adj::zsv<float>(), dB);
+  const float r[6] = {o.w.x, o.w.y, o.w.z, o.v.x, o.v.y, o.v.z};
+  memcpy(out, r, sizeof(r));
+  return SPI_OK;
+}
 // The equations-of-motion residual at the forward substep's accelerations (see hostemu_residual).
 int spi_hostemu_residual(const spi_robot* robot, const double* state, const double* theta, const double* act12,
                          double* out18) {

@@ -81,11 +81,18 @@ SPI_INL V3<T> contact_tan(const DevModel& M, T radius, T z, V3<T> v, V3<T> n, Co
   const T dfn = br.on ? -(T(M.k) * dz) - T(M.c) * (ds * vz + s * dvz) : T(0);
   dmimp = dmds * ds;
   const T dfz = dfn + dmimp * T(M.g);
+  // The branch is the forward pass's, vt is formed here, with other roundings: a slip's speed may come out as zero.
+  // Off, a slip has no friction whatever its speed; on, the value at rest is the sticking one.
   T scale = T(M.ct), dscale = T(0);
   if (!br.stick) {
-    const T inv = T(1) / m_sqrt(dot(vt, vt));
-    scale = T(M.mu) * fn * inv;
-    dscale = (T(M.mu) * dfn - scale * dot(vt, dvt) * inv) * inv;
+    const T vv = dot(vt, vt);
+    if (!br.on) {
+      scale = T(0);
+    } else if (vv > T(0)) {
+      const T inv = T(1) / m_sqrt(vv);
+      scale = T(M.mu) * fn * inv;
+      dscale = (T(M.mu) * dfn - scale * dot(vt, dvt) * inv) * inv;
+    }
   }
   return v3(dfz * n.x + fz * dn.x - dscale * vt.x - scale * dvt.x, dfz * n.y + fz * dn.y - dscale * vt.y - scale * dvt.y,
             dfz * n.z + fz * dn.z - dscale * vt.z - scale * dvt.z);
@@ -210,12 +217,9 @@ SPI_INL SV<T> corner_residual_tan(const DevModel& M, const BaseState<T>& B, V3<T
   const V3<T> vc = cross_acc(B.nu.w, rc, B.nu.v), dvc = cross_acc(dB.nu.w, rc, dB.nu.v);
   const V3<T> vw = mul(B.R, vc), dvw = mul(dB.R, vc) + mul(B.R, dvc);
   const T zc = B.p.z + dot(row(B.R, 2), rc), dz = dB.p.z + dot(row(dB.R, 2), rc);
-  T mc, dmc;
-  const V3<T> F = contact_force_local(M, T(0), zc, vw, ez, &mc);
-  ContactBranch br;
-  br.on = T(M.k) * (T(0) - zc) - T(M.c) * m_clamp((T(0) - zc) * T(M.ramp_inv), T(0), T(1)) * vw.z > T(0);
-  const T vtn = m_sqrt(vw.x * vw.x + vw.y * vw.y);
-  br.stick = !(T(M.ct) * vtn > T(M.mu) * (F.z - mc * T(M.g)));
+  T mc, dmc, branch[2];
+  const V3<T> F = contact_force_local(M, T(0), zc, vw, ez, &mc, branch);
+  const ContactBranch br = {branch[0] > T(0), branch[1] == T(M.ct)};
   const V3<T> dF = contact_tan(M, T(0), zc, vw, ez, br, dz, dvw, z0, dmc);
   const V3<T> dFb = mulT(dB.R, F) + mulT(B.R, dF);
   const V3<T> u = dmc * cross_acc(a0.w, rc, a0.v) - dFb;     // rate of the point's force

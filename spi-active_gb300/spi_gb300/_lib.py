@@ -115,6 +115,11 @@ def hostemu_lib():
         lib.spi_hostemu_tangent.restype = c_int
         lib.spi_hostemu_tangent.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
                                             c_void_p]
+        lib.spi_hostemu_contact_tan.restype = c_int
+        lib.spi_hostemu_contact_tan.argtypes = [POINTER(SpiRobot), c_float, c_void_p, c_void_p, c_int, c_int, c_float,
+                                                c_void_p, c_void_p, c_void_p]
+        lib.spi_hostemu_corner_tan.restype = c_int
+        lib.spi_hostemu_corner_tan.argtypes = [POINTER(SpiRobot), c_int, c_int, c_float, c_void_p, c_void_p, c_void_p]
         lib.spi_hostemu_residual.restype = c_int
         lib.spi_hostemu_residual.argtypes = [POINTER(SpiRobot), c_void_p, c_void_p, c_void_p, c_void_p]
         _hostemu = lib

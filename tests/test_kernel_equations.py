@@ -170,6 +170,58 @@ def test_substep_tangents_equal_central_differences(built, kw):
             assert np.linalg.norm(d - ref) <= 1e-4 * max(np.linalg.norm(ref), 1e-2), (b, k)
 
 
+def _f32p(*a):
+    return [np.ascontiguousarray(x, dtype=np.float32) for x in a]
+
+
+@pytest.mark.parametrize("vz", [-1.0, -0.5, 0.25])
+def test_contact_tangent_at_a_speed_that_rounds_to_zero(built, vz):
+    """The branch comes from the pass that produced the trajectory, the tangential velocity is formed again and
+    may come out as exactly zero where that pass saw some. A foot that is off and slipping has no friction
+    and none of its derivative; one that is on and slipping takes the sticking value, the model's at rest; one
+    that is sticking keeps its damping, on or off. All exact in these numbers."""
+    from spi_gb300 import _lib, robot
+    cfg = robot.SimConfig()
+    r, lib = robot.to_struct(cfg), _lib.hostemu_lib()
+    v, n, dv, dn = _f32p([0, 0, vz], [0, 0, 1], [1, 2, 0], [0, 0, 0])
+
+    def tan(z, on, stick):
+        out = np.zeros(4, dtype=np.float32)
+        assert lib.spi_hostemu_contact_tan(ctypes.byref(r), z, v.ctypes.data, n.ctypes.data, on, stick, 0.0,
+                                           dv.ctypes.data, dn.ctypes.data, out.ctypes.data) == 0
+        return out
+    ct = np.float32(r.contact_ct)
+    assert np.array_equal(tan(0.3, 0, 0), [0, 0, 0, 0])
+    assert np.array_equal(tan(0.3, 0, 1), [-ct, -2 * ct, 0, 0])
+    assert np.array_equal(tan(0.0, 1, 0), tan(0.0, 1, 1)) and np.isfinite(tan(0.0, 1, 1)).all()
+
+
+def test_corner_tangent_takes_the_force_models_branch(built):
+    """A base corner whose normal force (here some 1e-6 N) is far below its implicit mass's share of gravity (1e4 N), which
+    it is added to: sliding at 1e-13 m/s it sticks (ct v < mu f), so a change of the velocity along x changes
+    the force by -ct. The velocities leave a level base's other terms at zero, and ct is exact."""
+    from spi_gb300 import _lib, robot
+    r, lib = robot.to_struct(robot.SimConfig(contact_ct=2e6)), _lib.hostemu_lib()
+    pen = np.float32(0.5) * np.float32(r.contact_ramp)
+    corner = np.array(r.corners[0][:], dtype=np.float32)
+    z = np.float32(-pen - corner[2])
+    pen = float(np.float32(0) - np.float32(z + corner[2]))
+    s = float(np.float32(pen) * np.float32(1.0 / np.float32(r.contact_ramp)))
+    # a vertical velocity at which k pen and c s vz agree to within FP32 rounding, force just above zero
+    vz = np.float32(r.contact_k * pen / (r.contact_c * s))
+    for _ in range(64):
+        f = np.float32(np.float32(r.contact_k) * np.float32(pen)) - np.float32(np.float32(np.float32(r.contact_c) * np.float32(s)) * vz)
+        if f > 0:
+            break
+        vz = np.nextafter(vz, np.float32(0))
+    assert 0 < f < 1e-4
+    assert r.contact_ct * 1e-13 < r.contact_mu * f
+    v, dv = _f32p([1e-13, 0, vz], [1, 0, 0])
+    out = np.zeros(6, dtype=np.float32)
+    assert lib.spi_hostemu_corner_tan(ctypes.byref(r), 0, 0, float(z), v.ctypes.data, dv.ctypes.data, out.ctypes.data) == 0
+    assert out[3] == np.float32(r.contact_ct)
+
+
 def test_kernel_vs_oracle_with_urdf_constants(built):
     """Float32 model constants move states by < 1e-5 (well inside the 1e-4 parity bar)."""
     cfg, x0, acts, th = _inputs(13)
