@@ -150,6 +150,7 @@ int spi_create(const spi_robot* robot, spi_engine** out) {
   int dev = 0;
   ce = cudaGetDevice(&dev);
   if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, dev);
+  if (ce == cudaSuccess) ce = sensitivity_prepare();
   if (ce != cudaSuccess) { spi_destroy(e); return cuda_error(ce, "spi_create: device"); }
   // default kernel: the lane layout at the 168-register cap (the fastest on the C1 workload)
   if ((rc = spi_set_kernel_layout(e, SPI_LAYOUT_LANE)) || (rc = spi_set_kernel_config(e, 3))) {

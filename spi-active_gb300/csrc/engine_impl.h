@@ -43,5 +43,8 @@ int run_impl(spi_engine* e, float* trace);
 // them moved, drops the captured CEM graph and points the device CEM state at the new
 // theta / cost buffers.
 int refresh_after_realloc(spi_engine* e);
+// Raise the tangent kernels' dynamic shared-memory limit to what any number of directions needs. The limit belongs to
+// the kernel, not to an engine or a call: it is set to the same value by every engine, never per call.
+cudaError_t sensitivity_prepare();
 inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 }  // namespace spi

@@ -413,6 +413,12 @@ bool use_tangents(long long pairs, int K, int sms, int waves) {
   return K >= 3 && pairs * K > (long long)waves * 2 * 32 * sms;
 }
 
+// A CTA's staged pairs (32 consecutive quads touch so many at most) and its dynamic shared memory, bytes.
+int stage_pairs_of(int K) { return 31 / (K - 1) + 2; }
+int tangent_smem(int K, bool tapes) {
+  return stage_pairs_of(K) * (3 * kKeptFields + (tapes ? 8 * kTapeFields : 0)) * (int)sizeof(float4);
+}
+
 // Whether the tangents of a pair share one tape: with four or more to share it, and over two waves of the two
 // CTAs per SM that fit otherwise (H = 20, 152 SMs, whole call, own tapes against shared ones):
 //   4096 pairs x 13   1.69 / 1.55 ms      1650 x 13   1.06 / 1.00 ms      1530 x 13   0.86 / 0.92 ms
@@ -583,6 +589,17 @@ __global__ void __launch_bounds__(2 * kFisherThreads) fisher_kernel(const float*
 
 }  // namespace
 
+cudaError_t spi::sensitivity_prepare() {
+  int own = 0, shared = 0;
+  for (int K = 3; K <= SPI_THETA_DIM; ++K) {
+    own = std::max(own, tangent_smem(K, false));
+    shared = std::max(shared, tangent_smem(K, true));
+  }
+  const cudaError_t ce = cudaFuncSetAttribute(tangent_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, own);
+  if (ce != cudaSuccess) return ce;
+  return cudaFuncSetAttribute(tangent_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared);
+}
+
 extern "C" {
 
 int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* param_ids, int K, float* J, float* xH) {
@@ -611,14 +628,8 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
                      capture == cudaStreamCaptureStatusNone &&
                      e->sens_kept.reserve(slots * batch * kKeptBytes) == SPI_OK;
   if (!split) batch = all;
-  const int stage_pairs = split ? 31 / (K - 1) + 2 : 0;   // pairs that 32 consecutive quads can touch, at most
   const bool tapes = use_tapes(batch, K, e->sms);
-  const int smem = stage_pairs * (3 * kKeptFields + (tapes ? 8 * kTapeFields : 0)) * (int)sizeof(float4);
   const auto tangents = tapes ? tangent_kernel<true> : tangent_kernel<false>;
-  if (split) {
-    const cudaError_t fe = cudaFuncSetAttribute(tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (fe != cudaSuccess) return cuda_error(fe, "spi_sensitivity: shared memory");
-  }
   for (long long r0 = 0; r0 < all; r0 += batch) {
     a.nw0 = r0;
     a.nw = std::min(batch, all - r0);
@@ -626,7 +637,8 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
       a.legs = (float4*)e->sens_kept.p;
       a.base = a.legs + slots * kLegFields * 4 * a.nw;
       sensitivity_kernel<true><<<blocks_for(a.nw, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
-      tangents<<<blocks_for(a.nw * (K - 1), 32), 128, smem, e->stream>>>(e->d_model, win, theta, a, stage_pairs);
+      tangents<<<blocks_for(a.nw * (K - 1), 32), 128, tangent_smem(K, tapes), e->stream>>>(e->d_model, win, theta, a,
+                                                                                         stage_pairs_of(K));
     } else {
       sensitivity_kernel<false><<<blocks_for(a.nw * K, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
     }

@@ -1,0 +1,50 @@
+"""Engines used side by side on threads of one process."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import oracle_windows, random_theta
+
+pytestmark = pytest.mark.gpu
+
+
+def test_sensitivities_of_two_engines_on_two_threads(built):
+    """Five and thirteen directions, whose tangent kernels ask for different amounts of shared memory, in tight loops
+    of library calls: every call succeeds, and each engine's last result is its first to the bit."""
+    import ctypes
+
+    from spi_gb300.engine import Engine
+    from spi_gb300.robot import SimConfig
+    from spi_gb300.sensitivity import sensitivities
+    _, init, actions, target = oracle_windows(50, n_traj=2, T=160, H=1)
+    windows = [torch.from_numpy(a[:257]) for a in (init, actions, target)]
+    jobs = []
+    for N, ids in ((20, (0, 3, 7, 8, 12)), (8, tuple(range(13)))):
+        e = Engine(SimConfig(decimation=1), stream=torch.cuda.Stream())
+        e.load_windows(*windows)
+        th = torch.from_numpy(random_theta(np.random.default_rng(N), N).astype(np.float32)).cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(e.stream):
+            first = sensitivities(e, th, ids)[0]
+            jobs.append((e, th, ids, first, torch.zeros_like(first)))
+    torch.cuda.synchronize()
+    failures, gate = [], threading.Barrier(2)
+
+    def work(e, th, ids, first, J):
+        cids = (ctypes.c_int32 * len(ids))(*ids)
+        call = lambda: e.lib.spi_sensitivity(e._h, th.data_ptr(), th.shape[0], cids, len(ids), J.data_ptr(), None)  # noqa: E731
+        gate.wait(60)
+        for _ in range(100):
+            failures.extend((len(ids), rc) for rc in [call() for _ in range(100)] if rc)
+            e.stream.synchronize()
+        if not torch.equal(J, first):
+            failures.append((len(ids), "differs"))
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(200)
+    assert not any(t.is_alive() for t in threads)
+    assert not failures, (len(failures), failures[:5])
