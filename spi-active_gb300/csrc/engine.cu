@@ -165,6 +165,7 @@ int spi_destroy(spi_engine* e) {
   if (!e) return SPI_OK;
   if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
   if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
+  if (e->sens_done) cudaEventDestroy(e->sens_done);
   if (e->d_model) cudaFree(e->d_model);
   delete e;
   return SPI_OK;

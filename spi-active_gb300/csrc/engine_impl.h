@@ -34,6 +34,7 @@ struct spi_engine {
   cudaStream_t capture_stream = nullptr;   // graphs are captured here, replayed on `stream`
   unsigned seen_generation = 0;            // buffer generations the graph / CEM pointers refer to
   spi::DeviceBuf sens_kept;                // kept substeps of the sensitivities' first direction
+  cudaEvent_t sens_done = nullptr;         // after the last call that used sens_kept
   spi::DeviceBuf adj_ckpt, adj_seg, adj_part;   // adjoint checkpoints, kept substeps, partials
 };
 

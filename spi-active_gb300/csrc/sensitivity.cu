@@ -628,6 +628,13 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
                      capture == cudaStreamCaptureStatusNone &&
                      e->sens_kept.reserve(slots * batch * kKeptBytes) == SPI_OK;
   if (!split) batch = all;
+  // The results are the caller's and the directions' own rollouts share nothing, so calls on several streams
+  // (spi_set_stream) may overlap; the kept substeps are the engine's, and a call on another stream waits for them.
+  if (split) {
+    cudaError_t ce = e->sens_done ? cudaStreamWaitEvent(e->stream, e->sens_done, 0)
+                                  : cudaEventCreateWithFlags(&e->sens_done, cudaEventDisableTiming);
+    if (ce != cudaSuccess) return cuda_error(ce, "spi_sensitivity: order of the calls");
+  }
   const bool tapes = use_tapes(batch, K, e->sms);
   const auto tangents = tapes ? tangent_kernel<true> : tangent_kernel<false>;
   for (long long r0 = 0; r0 < all; r0 += batch) {
@@ -643,7 +650,8 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
       sensitivity_kernel<false><<<blocks_for(a.nw * K, 32), 128, 0, e->stream>>>(e->d_model, win, theta, a);
     }
   }
-  const cudaError_t ce = cudaGetLastError();
+  cudaError_t ce = cudaGetLastError();
+  if (ce == cudaSuccess && split) ce = cudaEventRecord(e->sens_done, e->stream);
   return ce == cudaSuccess ? SPI_OK : cuda_error(ce, "spi_sensitivity: launch");
 }
 

@@ -48,3 +48,31 @@ def test_sensitivities_of_two_engines_on_two_threads(built):
         t.join(200)
     assert not any(t.is_alive() for t in threads)
     assert not failures, (len(failures), failures[:5])
+
+
+def test_sensitivities_of_one_engine_on_two_streams(built):
+    """An engine moved from one stream to another between calls, nothing waiting in between: the calls' results
+    are those of each call alone, to the bit."""
+    import ctypes
+
+    from spi_gb300.engine import Engine
+    from spi_gb300.sensitivity import sensitivities
+    _, init, actions, target = oracle_windows(51, n_traj=2, T=160, H=5)
+    e = Engine()
+    e.load_windows(*(torch.from_numpy(a[:257]) for a in (init, actions, target)))
+    thetas = [torch.from_numpy(random_theta(np.random.default_rng(s), 8).astype(np.float32)).cuda() for s in (1, 2)]
+    alone = []
+    for th in thetas:
+        alone.append(sensitivities(e, th, range(13))[0])
+        torch.cuda.synchronize()
+    streams, ids = [torch.cuda.Stream() for _ in thetas], (ctypes.c_int32 * 13)(*range(13))
+    outs = [[torch.zeros_like(alone[0]) for _ in range(10)] for _ in thetas]
+    torch.cuda.synchronize()
+    for i in range(10):
+        for th, s, out in zip(thetas, streams, outs):
+            assert e.lib.spi_set_stream(e._h, ctypes.c_void_p(s.cuda_stream)) == 0
+            assert e.lib.spi_sensitivity(e._h, th.data_ptr(), 8, ids, 13, out[i].data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    e.lib.spi_set_stream(e._h, ctypes.c_void_p(e.stream.cuda_stream))
+    for out, ref in zip(outs, alone):
+        assert all(torch.equal(o, ref) for o in out)
