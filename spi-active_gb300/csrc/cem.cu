@@ -136,6 +136,7 @@ int spi_cem_step(spi_engine* e) {
 int spi_cem_run(spi_engine* e, int iterations, int use_graph) {
   if (!e || !e->cem_ready) return set_error(SPI_ESTATE, "spi_cem_run before spi_cem_init");
   if (iterations < 0) return set_error(SPI_EINVAL, "spi_cem_run: iterations < 0");
+  if (iterations == 0) return SPI_OK;
   if (!use_graph) {
     for (int i = 0; i < iterations; ++i) {
       int rc = cem_step_impl(e);
@@ -143,6 +144,12 @@ int spi_cem_run(spi_engine* e, int iterations, int use_graph) {
     }
     return SPI_OK;
   }
+  // what the captured step sets and asks for outside the device's work: the engine's batch is the population again
+  // (an evaluation may have come in between), with room for its run
+  e->N = e->cem_n;
+  e->population = true;
+  int rc = reserve_run(e);
+  if (rc) return rc;
   if (!e->graph_exec) {
     // capture one iteration on a private stream (the engine stream may be the legacy
     // default stream, which cannot be captured), replay it on the engine stream
@@ -155,7 +162,7 @@ int spi_cem_run(spi_engine* e, int iterations, int use_graph) {
     e->stream = e->capture_stream;
     cudaError_t ce = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
     if (ce != cudaSuccess) { e->stream = user; return cuda_error(ce, "spi_cem_run: begin capture"); }
-    int rc = cem_step_impl(e);
+    rc = cem_step_impl(e);
     ce = cudaStreamEndCapture(e->stream, &g);
     e->stream = user;
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }

@@ -53,22 +53,22 @@ __global__ void finalize_evaluate(const float* __restrict__ partial, int N, int 
   if (cost) cost[n] = own_cost[n];
 }
 
-// The buffers of a run over the engine's theta batch.
-int reserve_run(spi_engine* e, int G) {
+}  // namespace
+
+int spi::reserve_run(spi_engine* e) {
+  const int G = (e->W + 7) / 8;
   int rc = e->partial.reserve((size_t)e->N * G * SPI_N_COMP * sizeof(float));
   if (!rc) rc = e->comp.reserve((size_t)e->N * SPI_N_COMP * sizeof(float));
   if (!rc) rc = e->cost.reserve((size_t)e->N * sizeof(float));
   return rc ? rc : refresh_after_realloc(e);
 }
 
-}  // namespace
-
 int spi::run_impl(spi_engine* e, float* trace) {
   if (!e) return set_error(SPI_EINVAL, "null engine");
   if (e->W <= 0 || e->H <= 0) return set_error(SPI_ESTATE, "spi_run before spi_load_windows");
   if (e->N <= 0) return set_error(SPI_ESTATE, "spi_run before spi_set_theta");
   const int G = (e->W + 7) / 8;
-  int rc = reserve_run(e, G);
+  int rc = reserve_run(e);
   if (rc) return rc;
   WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
   const long long warps = (long long)e->N * G;
@@ -268,7 +268,7 @@ int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* c
   e->N = N;
   e->population = false;
   e->ran = false;
-  if ((rc = reserve_run(e, G))) return rc;
+  if ((rc = reserve_run(e))) return rc;
   const WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
   const EvalArgs a{win, theta, e->partial.f(), N, G, (unsigned long long*)e->bad.p};
   cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);

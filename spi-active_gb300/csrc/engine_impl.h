@@ -40,6 +40,8 @@ struct spi_engine {
 
 namespace spi {
 int run_impl(spi_engine* e, float* trace);
+// The buffers of a run over the engine's theta batch; what depends on their addresses follows them.
+int reserve_run(spi_engine* e);
 // Call after any DeviceBuf::reserve of theta / cost / partial / comp / windows: if one of
 // them moved, drops the captured CEM graph and points the device CEM state at the new
 // theta / cost buffers.

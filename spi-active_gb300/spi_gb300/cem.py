@@ -75,6 +75,7 @@ class CEM:
         """One iteration: sample, roll every (theta, window), refit. Events bracket the rollout."""
         h = self.engine._h
         _lib.check(self.lib.spi_cem_sample(h))
+        self.engine.N = self.cfg.n_samples   # the engine's batch is the population
         if rollout_events:
             rollout_events[0].record(self.engine.stream)
         _lib.check(self.engine.lib.spi_run(h))
@@ -84,12 +85,15 @@ class CEM:
 
     def sample(self):
         _lib.check(self.lib.spi_cem_sample(self.engine._h))
+        self.engine.N = self.cfg.n_samples
 
     def refit(self):
         _lib.check(self.lib.spi_cem_refit(self.engine._h))
 
     def run(self, iterations, graph=True):
         _lib.check(self.lib.spi_cem_run(self.engine._h, int(iterations), int(bool(graph))))
+        if iterations:
+            self.engine.N = self.cfg.n_samples
 
     def read(self):
         P = len(self.param_ids)
