@@ -17,14 +17,14 @@ int cuda_error(cudaError_t e, const char* what);
 struct DeviceBuf {
   void* p = nullptr;
   size_t cap = 0;
-  unsigned generation = 0;   // bumped whenever the allocation moves
+  unsigned generation = 0;   // bumped whenever the allocation moves or goes
   DeviceBuf() = default;
   DeviceBuf(const DeviceBuf&) = delete;
   DeviceBuf& operator=(const DeviceBuf&) = delete;
   ~DeviceBuf() { if (p) cudaFree(p); }
   int reserve(size_t bytes) {
     if (bytes <= cap) return SPI_OK;
-    if (p) { cudaFree(p); p = nullptr; cap = 0; }
+    if (p) { cudaFree(p); p = nullptr; cap = 0; ++generation; }
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();

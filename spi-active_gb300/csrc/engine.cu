@@ -53,6 +53,13 @@ __global__ void finalize_evaluate(const float* __restrict__ partial, int N, int 
   if (cost) cost[n] = own_cost[n];
 }
 
+// Room for N theta samples. Without it the batch that the engine had is gone too.
+int reserve_theta(spi_engine* e, int N) {
+  const int rc = e->theta.reserve((size_t)N * SPI_THETA_DIM * 4);
+  if (rc) { e->N = 0; e->ran = false; }
+  return rc;
+}
+
 }  // namespace
 
 int spi::reserve_run(spi_engine* e) {
@@ -60,6 +67,7 @@ int spi::reserve_run(spi_engine* e) {
   int rc = e->partial.reserve((size_t)e->N * G * SPI_N_COMP * sizeof(float));
   if (!rc) rc = e->comp.reserve((size_t)e->N * SPI_N_COMP * sizeof(float));
   if (!rc) rc = e->cost.reserve((size_t)e->N * sizeof(float));
+  if (rc) e->ran = false;   // a buffer that could not grow is gone
   return rc ? rc : refresh_after_realloc(e);
 }
 
@@ -203,7 +211,7 @@ int spi_load_windows(spi_engine* e, const float* init, const float* actions, con
 int spi_set_theta(spi_engine* e, const float* theta, int N) {
   if (!e || !theta) return set_error(SPI_EINVAL, "spi_set_theta: null argument");
   if (N <= 0) return set_error(SPI_EINVAL, "spi_set_theta: N=%d must be > 0", N);
-  int rc = e->theta.reserve((size_t)N * SPI_THETA_DIM * 4);
+  int rc = reserve_theta(e, N);
   if (rc) return rc;
   if ((rc = refresh_after_realloc(e))) return rc;
   cudaError_t ce = cudaMemcpyAsync(e->theta.p, theta, (size_t)N * SPI_THETA_DIM * 4,
@@ -263,12 +271,16 @@ int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* c
     return rc ? rc : spi_read_costs(e, comp, cost);
   }
   const int G = (e->W + 7) / 8;
-  int rc = e->theta.reserve((size_t)N * SPI_THETA_DIM * 4);
+  int rc = reserve_theta(e, N);
   if (rc) return rc;
   e->N = N;
   e->population = false;
   e->ran = false;
-  if ((rc = reserve_run(e))) return rc;
+  if ((rc = reserve_run(e))) {
+    // no room for the run: the batch is set all the same, as by spi_set_theta before a spi_run that finds none
+    cudaMemcpyAsync(e->theta.p, theta, (size_t)N * SPI_THETA_DIM * 4, cudaMemcpyDeviceToDevice, e->stream);
+    return rc;
+  }
   const WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
   const EvalArgs a{win, theta, e->partial.f(), N, G, (unsigned long long*)e->bad.p};
   cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);

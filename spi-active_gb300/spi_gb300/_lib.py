@@ -11,7 +11,7 @@ from ctypes import POINTER, c_double, c_float, c_int, c_int64, c_void_p
 from ._build import ENGINE_SO, HOSTEMU_SO
 from .robot import SpiRobot
 
-SPI_OK = 0
+SPI_OK, SPI_EINVAL, SPI_ENOMEM, SPI_ESTATE = 0, -1, -2, -4
 ERRORS = {-1: "SPI_EINVAL", -2: "SPI_ENOMEM", -3: "SPI_ECUDA", -4: "SPI_ESTATE",
           -5: "SPI_ETIMEOUT", -6: "SPI_EBUDGET"}
 

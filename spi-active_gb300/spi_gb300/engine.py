@@ -125,9 +125,11 @@ class Engine:
         N = theta.shape[0]
         comp = torch.empty((N, N_COMP), device=self.device)
         cost = torch.empty((N,), device=self.device)
-        _lib.check(self.lib.spi_evaluate(self._h, theta.data_ptr(), N, comp.data_ptr(), cost.data_ptr()))
-        self._theta = theta
-        self.N = N
+        rc = self.lib.spi_evaluate(self._h, theta.data_ptr(), N, comp.data_ptr(), cost.data_ptr())
+        if rc not in (_lib.SPI_EINVAL, _lib.SPI_ESTATE):   # the batch is set, also where the run found no memory
+            self._theta = theta
+            self.N = N
+        _lib.check(rc)
         return comp, cost
 
 

@@ -46,3 +46,50 @@ def test_evaluation_between_cem_runs(built, graph):
     assert a[0].shape == (64, 13) and all(torch.equal(x, y) for x, y in zip(a[:3], b[:3]))
     assert torch.equal(a[1], a[2])
     assert a[3]["best_cost"] == b[3]["best_cost"] and np.array_equal(a[3]["mu"], b[3]["mu"])
+
+
+def _too_many(W):
+    """Theta samples whose window-group results (36 bytes each) no GPU holds: 300,000 of 32,768 groups, 354 GB."""
+    assert W == 32768 * 8
+    return torch.from_numpy(random_theta(np.random.default_rng(2), 300).astype(np.float32)).repeat(1000, 1)
+
+
+def _many_windows():
+    w = [a[:1].repeat(32768 * 8, *([1] * (a.ndim - 1))) for a in _windows(19, H=1)]
+    return w
+
+
+def test_evaluation_without_memory_leaves_the_batch(built):
+    """An evaluation that finds no memory fails as spi_set_theta and a failing spi_run do: the batch is the caller's,
+    and runs once the windows are fewer."""
+    from spi_gb300 import _lib
+    few, th = _windows(8, H=1), _too_many(32768 * 8)
+    e = _engine(_many_windows())
+    e.evaluate(th[:2])
+    with pytest.raises(_lib.SpiError) as err:
+        e.evaluate(th)
+    assert err.value.code == _lib.SPI_ENOMEM
+    with pytest.raises(_lib.SpiError):
+        e.read()
+    e.load_windows(*few)
+    e.run()
+    cost = e.read()[1]
+    assert cost.shape == (300000,) and torch.equal(cost, _engine(few).evaluate(th)[1])
+
+
+def test_cem_after_an_evaluation_without_memory(built):
+    """The failed evaluation has moved buffers that the captured CEM step refers to; the next run is still that of a
+    CEM without it, to the bit."""
+    from spi_gb300 import _lib
+    windows, got = _many_windows(), []
+    for fail in (False, True):
+        e = _engine(windows)
+        cem = _cem(e, n=4)
+        cem.run(2)
+        if fail:
+            with pytest.raises(_lib.SpiError):
+                e.evaluate(_too_many(32768 * 8))
+        cem.run(1)
+        got.append((cem.theta(), e.read()[1], cem.read()["best_cost"]))
+        e.close()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2]
