@@ -470,25 +470,6 @@ template <int AX, int RM, class T> SPI_INL void ri_to_parent_art_acc(const RI<T>
 struct alignas(16) F4 { float x, y, z, w; };
 constexpr int kLegSlots = 14;
 
-// A leg's constants as leg_condense (leg_hip.cuh) reads them, four to a 16-byte slot; 13 slots, so that the four legs' copies of a slot
-// start in different shared-memory banks.
-template <class S> struct alignas(16) HipLeg {
-  S x0, y0, y1, z2;            // hip origin (x0, y0, 0), thigh origin (0, y1, 0), calf origin (0, 0, z2)
-  S kd[3], m0;                 // joint damping; hip mass
-  S iv[3], m12;                // 1 / velocity limit (0: no limit); thigh + calf mass
-  S h0x, h0y, h0z, m2;         // hip first moment; calf mass
-  S J0xx, J0yy, J0zz, J0xy;    // hip second moments about o0
-  S J0xz, J0yz, h1x, h1z;      // thigh about o0, thigh axes: first moment,
-  S h1y, P1, D1, X1;           //   (Jxx + Jzz) / 2, (Jxx - Jzz) / 2, Jxz,
-  S J1xy, J1yz, yy12, h2x;     //   Jxy, Jyz; Jyy of thigh (about o0) + calf (about its joint)
-  S h2y, h2z, P2, D2;          // calf about its joint, calf axes: as the thigh
-  S X2, J2xy, J2yz, hf2;       //   hf2 = (foot z)^2 / 2
-  S c0x, c0y, c0z, c1x;        // the leg's two base-box corners
-  S c1y, c1z, pad[2];
-  S pad2[4];
-};
-static_assert(sizeof(HipLeg<float>) == 13 * 16, "HipLeg: 13 slots");
-
 struct DevModel {
   // The per-leg constants phase A reads, leg-major, four to a 16-byte slot, so that one leg's
   // are contiguous (one 128-bit load per slot) and the four legs' copies of a slot sit 56
@@ -498,7 +479,6 @@ struct DevModel {
   //          (1 / vlim is 0 without the torque-speed limit)
   //   12, 13 the leg's two base-box corners: (c0 x, c0 y, c0 z, c1 x), (c1 y, c1 z, 0, 0)
   F4 legc[4][kLegSlots];
-  HipLeg<float> hip[4];
   // per leg body k (0 hip, 1 thigh, 2 calf), component, leg: [k][c][leg] (the same constants
   // as the source arrays of legc, for the host-side formulations)
   float org[3][3][4];

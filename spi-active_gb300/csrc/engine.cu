@@ -145,11 +145,11 @@ int spi_create(const spi_robot* robot, spi_engine** out) {
   spi_engine* e = new (std::nothrow) spi_engine();
   if (!e) return set_error(SPI_ENOMEM, "spi_create: host allocation failed");
   const char* why = "";
-  int rc = build_dev_model(*robot, &e->host_model, &why);
+  int rc = build_eval_model(*robot, &e->host_model, &why);
   if (rc) { delete e; return set_error(rc, "spi_create: %s", why); }
   cudaError_t ce = cudaMalloc(&e->d_model, sizeof(DevModel));
   if (ce != cudaSuccess) { delete e; return cuda_error(ce, "spi_create: cudaMalloc(model)"); }
-  ce = cudaMemcpy(e->d_model, &e->host_model, sizeof(DevModel), cudaMemcpyHostToDevice);
+  ce = cudaMemcpy(e->d_model, static_cast<const DevModel*>(&e->host_model), sizeof(DevModel), cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) { cudaFree(e->d_model); delete e; return cuda_error(ce, "spi_create: upload model"); }
   rc = e->bad.reserve(sizeof(unsigned long long));
   if (!rc) rc = e->items.reserve(sizeof(SingleTable));

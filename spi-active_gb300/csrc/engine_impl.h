@@ -5,10 +5,10 @@
 
 #include "cem_state.h"
 #include "common.h"
-#include "dynamics.cuh"
+#include "leg_hip.cuh"
 
 struct spi_engine {
-  spi::DevModel host_model;
+  spi::EvalModel host_model;
   spi::DevModel* d_model = nullptr;
   int sms = 0;                             // SMs of the engine's device
   cudaStream_t stream = nullptr;

@@ -18,7 +18,7 @@ namespace {
 // used, the FP32 pipe 66 % busy. 4096 theta x 256 windows x H = 20: 7.87 ms; 8.92 ms with phase A of
 // dynamics.cuh (3,710 instructions).
 template <int MINB, int MS>
-__global__ void __launch_bounds__(128, MINB) eval_lane_kernel(const __grid_constant__ DevModel M, const EvalArgs a) {
+__global__ void __launch_bounds__(128, MINB) eval_lane_kernel(const __grid_constant__ EvalModel M, const EvalArgs a) {
   extern __shared__ float4 lane_smem[];              // kHipSlotBytes
   __shared__ BaseParams<float> bp_warp[4][4];
   __shared__ float4 gains_warp[4][4][8];
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(128, MINB) eval_lane_kernel(const __grid_const
 // Latency-bound: one chain of substeps per rollout, at most a few warps per scheduler. 64 theta x 8 windows
 // x H = 5: 26 us for the launch and its finalize, against 57 us with one lane per rollout.
 template <int MS>
-__global__ void __launch_bounds__(128) eval_team_kernel(const __grid_constant__ DevModel M, const EvalArgs a) {
+__global__ void __launch_bounds__(128) eval_team_kernel(const __grid_constant__ EvalModel M, const EvalArgs a) {
   __shared__ TeamShare share_cta[4];
   __shared__ HipLeg<float> hip[4];
   stage_hip(hip, M);
@@ -150,7 +150,7 @@ cudaError_t eval_prepare() {
   return cudaSuccess;
 }
 
-cudaError_t eval_launch(const DevModel& model, int min_blocks, int sms, const EvalArgs& a, cudaStream_t stream) {
+cudaError_t eval_launch(const EvalModel& model, int min_blocks, int sms, const EvalArgs& a, cudaStream_t stream) {
   const bool sl = motor_shape_of(model) == kMotorSpeedLimit;
   const long long pairs = (long long)a.N * a.G;
   const void* func;

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "leg_hip.cuh"
 #include "rollout.cuh"
 
 namespace spi {
@@ -18,6 +19,6 @@ struct EvalArgs {
 // Raise the dynamic shared-memory limit of the lane-form kernels.
 cudaError_t eval_prepare();
 // Launch the rollouts of `a` on a GPU of `sms` SMs. min_blocks 2..4: the lane form's register cap.
-cudaError_t eval_launch(const DevModel& model, int min_blocks, int sms, const EvalArgs& a, cudaStream_t stream);
+cudaError_t eval_launch(const EvalModel& model, int min_blocks, int sms, const EvalArgs& a, cudaStream_t stream);
 
 }  // namespace spi

@@ -21,6 +21,33 @@
 
 namespace spi {
 
+// A leg's constants as leg_condense reads them, four to a 16-byte slot; 13 slots, so that the four legs' copies of a slot
+// start in different shared-memory banks.
+template <class S> struct alignas(16) HipLeg {
+  S x0, y0, y1, z2;            // hip origin (x0, y0, 0), thigh origin (0, y1, 0), calf origin (0, 0, z2)
+  S kd[3], m0;                 // joint damping; hip mass
+  S iv[3], m12;                // 1 / velocity limit (0: no limit); thigh + calf mass
+  S h0x, h0y, h0z, m2;         // hip first moment; calf mass
+  S J0xx, J0yy, J0zz, J0xy;    // hip second moments about o0
+  S J0xz, J0yz, h1x, h1z;      // thigh about o0, thigh axes: first moment,
+  S h1y, P1, D1, X1;           //   (Jxx + Jzz) / 2, (Jxx - Jzz) / 2, Jxz,
+  S J1xy, J1yz, yy12, h2x;     //   Jxy, Jyz; Jyy of thigh (about o0) + calf (about its joint)
+  S h2y, h2z, P2, D2;          // calf about its joint, calf axes: as the thigh
+  S X2, J2xy, J2yz, hf2;       //   hf2 = (foot z)^2 / 2
+  S c0x, c0y, c0z, c1x;        // the leg's two base-box corners
+  S c1y, c1z, pad[2];
+  S pad2[4];
+};
+static_assert(sizeof(HipLeg<float>) == 13 * 16, "HipLeg: 13 slots");
+
+// The model of the evaluation kernels, by value in their parameter block. The legs' constants stay out of DevModel: every
+// other kernel copies that one to shared memory, CTA by CTA (832 bytes more took step_kernel, four substeps long,
+// from 8.3 to 8.9 us).
+struct EvalModel : DevModel {
+  HipLeg<float> hip[4];
+};
+static_assert(sizeof(DevModel) == 2064, "DevModel: what every CTA copies");
+
 // The constants of `leg` from the public robot description (S = float on the device).
 template <class S> inline HipLeg<S> hip_leg_constants(const spi_robot& r, int leg) {
   HipLeg<S> c = {};

@@ -88,11 +88,17 @@ inline int build_dev_model(const spi_robot& r, DevModel* M, const char** why) {
     *why = "sim_dt must be > 0 and decimation in [1, 64]"; return SPI_EINVAL;
   }
   if (!(r.friction_vel > 0.0f)) { *why = "friction_vel must be > 0"; return SPI_EINVAL; }
-  for (int leg = 0; leg < 4; ++leg) M->hip[leg] = hip_leg_constants<float>(r, leg);
   M->fric_k2 = (float)(2.0 / (log(2.0) * (double)r.friction_vel));
   if (r.inertia_follows_mass && !(r.base_mass_nominal > 0.0f)) {
     *why = "base_mass_nominal must be > 0 with inertia_follows_mass"; return SPI_EINVAL;
   }
+  return SPI_OK;
+}
+
+inline int build_eval_model(const spi_robot& r, EvalModel* M, const char** why) {
+  const int rc = build_dev_model(r, M, why);
+  if (rc) return rc;
+  for (int leg = 0; leg < 4; ++leg) M->hip[leg] = hip_leg_constants<float>(r, leg);
   return SPI_OK;
 }
 

@@ -138,7 +138,7 @@ struct HipSlots {
 // One physics substep of one rollout on one lane. s: this thread's slots; bp: the warp's base
 // parameters; gains: the warp's four legs' LegGains (two fields each); pe: the base position's error.
 template <int MS>
-__device__ __forceinline__ void substep_hip_lane(const DevModel& M, BaseState<float>& B, V3<float>& pe, const HipSlots& s,
+__device__ __forceinline__ void substep_hip_lane(const EvalModel& M, BaseState<float>& B, V3<float>& pe, const HipSlots& s,
                                                  const BaseParams<float>* bp, const float4* gains) {
   // articulated inertia and bias force at the base: the base body's own, then each leg's in turn
   LegOut<float> sum = base_terms(*bp, B);
@@ -275,7 +275,7 @@ __device__ __forceinline__ LegOut<float> team_sum(TeamShare& share, const LegOut
 }
 
 // The legs' constants to shared memory (the lanes of a team index them by leg); the whole CTA.
-__device__ __forceinline__ void stage_hip(HipLeg<float> hip[4], const DevModel& M) {
+__device__ __forceinline__ void stage_hip(HipLeg<float> hip[4], const EvalModel& M) {
   if (threadIdx.x < 4 * sizeof(HipLeg<float>) / 16)
     reinterpret_cast<float4*>(hip)[threadIdx.x] = reinterpret_cast<const float4*>(M.hip)[threadIdx.x];
   __syncthreads();
