@@ -237,8 +237,7 @@ __device__ __forceinline__ void finalize_one(const float* __restrict__ partial, 
   float c[SPI_N_COMP];
 #pragma unroll
   for (int k = 0; k < SPI_N_COMP; ++k) c[k] = 0.f;
-#pragma unroll 8
-  for (int g = 0; g < G; ++g) {   // the sums in order, the loads of eight groups in flight
+  for (int g = 0; g < G; ++g) {
     const float* p = partial + ((size_t)n * G + g) * SPI_N_COMP;
 #pragma unroll
     for (int k = 0; k < SPI_N_COMP; ++k) c[k] = __fadd_rn(c[k], p[k]);
