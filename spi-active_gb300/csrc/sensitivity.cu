@@ -434,8 +434,10 @@ bool use_tapes(long long pairs, int K, int sms) {
 // these are summed), into shared memory in the layout the accumulation reads; the sums run from there
 // in row order, as one chain per entry (FP32) or per 8-column tile of the m16n8k16 product (tensor
 // cores), so the staging does not show in a result. The scores follow in the same launch, both
-// samples on one warp: an FP64 instruction holds GB300's FP64 pipe for sixteen cycles whatever its
-// lanes do, and a sample has 13 rows. 512 samples x 8 windows x 13 parameters, BF16: 115 -> 16.5 us.
+// samples on one warp (a sample has 13 rows at most, and an FP64 instruction takes as long for one
+// lane as for 32). 512 samples x 8 windows x 13 parameters, BF16: 115 -> 16.5 us. For many samples the
+// scores, and of few windows the sums too, come from kernels with less fixed work a sample (many_samples,
+// few_rows below); a sample's results are the same to the bit by each.
 // ---------------------------------------------------------------------------
 constexpr int kFisherRows = 128;                 // rows of J staged at a time (a multiple of 16)
 constexpr int kFisherPitch = kFisherRows / 2 + 4;   // words per parameter of the BF16 tile; 4 mod 32: conflict-free
@@ -465,7 +467,7 @@ __device__ __forceinline__ void fisher_scores(const float* F, int K, double eps,
       const double l = row[j] * (1.0 / d);
 #pragma unroll
       for (int k = j + 1; k < SPI_THETA_DIM; ++k)
-        if (k < K) row[k] -= l * __shfl_sync(0xffffffffu, row[j], k, 16);
+        if (k < K) row[k] = fma(-l, __shfl_sync(0xffffffffu, row[j], k, 16), row[k]);
     }
   }
   const double lg = log(pivot);
@@ -477,6 +479,40 @@ __device__ __forceinline__ void fisher_scores(const float* F, int K, double eps,
   }
 }
 
+// The same, in the same operations, from F in memory with one sample a thread, for many samples: a warp's FP64
+// instruction then serves 32 samples (fisher_scores: two), but a sample is one thread's chain. The lower
+// triangle is in registers.
+__global__ void __launch_bounds__(32) fisher_scores_kernel(const float* __restrict__ F, int N, int K, double eps,
+                                                           double* __restrict__ logdet, double* __restrict__ trace) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const float* f = F + (size_t)n * K * K;
+  double A[SPI_THETA_DIM][SPI_THETA_DIM];
+#pragma unroll
+  for (int i = 0; i < SPI_THETA_DIM; ++i)
+#pragma unroll
+    for (int j = 0; j <= i; ++j) A[i][j] = i < K ? (double)f[i * K + j] + (j == i ? eps : 0.0) : 0.0;
+  double ld = 0.0, tr = 0.0;
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < SPI_THETA_DIM; ++j) {
+    if (j >= K) break;                            // uniform
+    if (ok) tr += (double)f[j * K + j];
+    const double d = A[j][j];
+    ok = ok && d > 0.0;
+    ld += log(d);
+    const double inv = 1.0 / d;
+#pragma unroll
+    for (int i = j + 1; i < SPI_THETA_DIM; ++i)
+      if (i < K) {
+        const double l = A[i][j] * inv;
+#pragma unroll
+        for (int k = j + 1; k <= i; ++k) A[i][k] = fma(-l, A[k][j], A[i][k]);
+      }
+  }
+  if (logdet) logdet[n] = ok ? ld : -INFINITY;
+  if (trace) trace[n] = tr;
+}
 // TC = false: FP32 on the CUDA cores, one entry (p, r >= p) a thread: acc += (q J_p) J_r over the rows.
 // TC = true: BF16 operands (Q^1/2 J), FP32 accumulation, mma.sync m16n8k16 by one warp: A = (Q^1/2 J)^T
 // as a 16 x 16 tile, B = Q^1/2 J as two 16 x 8 tiles (the same registers: A's row groups are B's columns).
@@ -587,6 +623,76 @@ __global__ void __launch_bounds__(2 * kFisherThreads) fisher_kernel(const float*
   }
 }
 
+// The sums of fisher_kernel, in its order, for many samples of few rows: one warp a sample, straight from memory. Staging a
+// CTA's tile takes the same instructions however few rows there are.
+__device__ __forceinline__ unsigned jq_pair(const float* Jn, const float* q, int rows, int K, int r, int p) {
+  float v[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    v[i] = r + i < rows && p < K ? (q ? sqrtf(q[(r + i) % SPI_STATE_DIM]) : 1.f) * Jn[(size_t)(r + i) * K + p] : 0.f;
+  const __nv_bfloat162 b = __floats2bfloat162_rn(v[0], v[1]);
+  return *reinterpret_cast<const unsigned*>(&b);
+}
+template <bool TC>
+__global__ void __launch_bounds__(128) fisher_few_rows_kernel(const float* __restrict__ J, int N, int W, int K,
+                                                              const float* __restrict__ q, float* __restrict__ F) {
+  const int n = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (n >= N) return;                             // uniform per warp
+  const int lane = threadIdx.x & 31, rows = W * SPI_STATE_DIM;
+  const float* Jn = J + (size_t)n * rows * K;
+  float* Fn = F + (size_t)n * K * K;
+  if (TC) {
+    const int g = lane >> 2, t = lane & 3;
+    float c[2][4] = {};
+    for (int k0 = 0; k0 < rows; k0 += 16) {
+      const int r = k0 + 2 * t;
+      const unsigned a0 = jq_pair(Jn, q, rows, K, r, g), a1 = jq_pair(Jn, q, rows, K, r, g + 8),
+                     a2 = jq_pair(Jn, q, rows, K, r + 8, g), a3 = jq_pair(Jn, q, rows, K, r + 8, g + 8);
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+            "{%0, %1, %2, %3};\n"
+            : "+f"(c[nt][0]), "+f"(c[nt][1]), "+f"(c[nt][2]), "+f"(c[nt][3])
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(nt ? a1 : a0), "r"(nt ? a3 : a2));
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = g + (e >= 2 ? 8 : 0), j = 8 * nt + 2 * t + (e & 1);
+        if (i < K && j < K) Fn[i * K + j] = c[nt][e];
+      }
+  } else {
+    for (int e = lane; e < K * (K + 1) / 2; e += 32) {
+      int p = 0, r = e;
+      while (r >= K - p) { r -= K - p; ++p; }
+      r += p;
+      float acc = 0.f;
+      for (const float* Jw = Jn; Jw < Jn + rows * K; Jw += SPI_STATE_DIM * K) {
+#pragma unroll
+        for (int i = 0; i < SPI_STATE_DIM; ++i)
+          acc = fmaf((q ? __ldg(q + i) : 1.f) * __ldg(Jw + i * K + p), __ldg(Jw + i * K + r), acc);
+      }
+      Fn[p * K + r] = acc;
+      Fn[r * K + p] = acc;
+    }
+  }
+}
+
+// Whether the scores come in a launch of their own: a sample's take one chain's length then (6 us at K = 1, 38 at
+// K = 13), and up to some number of samples the half-warps are done first; FP32 sums of more windows
+// hide more of them. us a call, scores in the sums' launch / apart (sums by the better kernel):
+//   tensor cores  4096 x 1 x 13  60 / 52    4096 x 8 x 13  76 / 74    3000 x 8 x 8  45 / 46    50000 x 1 x 13  602 / 216
+//   FP32          4096 x 1 x 5   25 / 25    6000 x 1 x 13  60 / 62    8192 x 8 x 8  89 / 91    50000 x 1 x 5   222 / 99
+bool many_samples(int N, int W, int K, bool tc) {
+  return tc ? N > 1700 + 180 * K : (long long)N * 8 > (3000LL + 300 * K) * (8 + W);
+}
+// Whether the sums of many samples are by fisher_few_rows_kernel (us a call, staged / this one):
+//   tensor cores  16384 x 1 x 13  93 / 66    16384 x 4 x 5   82 / 62    16384 x 4 x 13  127 / 126    16384 x 8 x 13  160 / 172
+//   FP32          16384 x 1 x 1   38 / 21    16384 x 2 x 5   58 / 50    16384 x 1 x 13   93 / 87     50000 x 4 x 5   233 / 288
+bool few_rows(int W, int K, bool tc) { return tc ? W <= 4 : W * K <= 10; }
+
 }  // namespace
 
 cudaError_t spi::sensitivity_prepare() {
@@ -665,10 +771,16 @@ int spi_fisher_ex(const float* J, int N, int W, int K, const float* state_weight
   if (!J || !F || N <= 0 || W <= 0 || K < 1 || K > SPI_THETA_DIM)
     return set_error(SPI_EINVAL, "spi_fisher: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
-  if (tensor_cores)
-    fisher_kernel<true><<<(N + 1) / 2, 2 * kFisherThreads, 0, s>>>(J, N, W, K, state_weight, eps, F, logdet, trace);
-  else
-    fisher_kernel<false><<<(N + 1) / 2, 2 * kFisherThreads, 0, s>>>(J, N, W, K, state_weight, eps, F, logdet, trace);
+  const bool scores = logdet || trace, many = many_samples(N, W, K, tensor_cores != 0);
+  if (many && few_rows(W, K, tensor_cores != 0)) {
+    const auto kernel = tensor_cores ? fisher_few_rows_kernel<true> : fisher_few_rows_kernel<false>;
+    kernel<<<blocks_for(N, 4), 128, 0, s>>>(J, N, W, K, state_weight, F);
+  } else {
+    const auto kernel = tensor_cores ? fisher_kernel<true> : fisher_kernel<false>;
+    kernel<<<blocks_for(N, 2), 2 * kFisherThreads, 0, s>>>(J, N, W, K, state_weight, eps, F, many ? nullptr : logdet,
+                                                          many ? nullptr : trace);
+  }
+  if (many && scores) fisher_scores_kernel<<<blocks_for(N, 32), 32, 0, s>>>(F, N, K, eps, logdet, trace);
   cudaError_t ce = cudaGetLastError();
   return ce == cudaSuccess ? SPI_OK : cuda_error(ce, "spi_fisher");
 }

@@ -28,3 +28,25 @@ def test_fisher_equals_fp64(built, N, W, K, tensor_cores):
     eye = 1e-6 * torch.eye(K, device="cuda", dtype=torch.float64)
     assert torch.allclose(logdet, torch.logdet(own + eye), rtol=1e-9, atol=1e-9)
     assert torch.allclose(trace, torch.diagonal(own, dim1=1, dim2=2).sum(-1), rtol=1e-12)
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+@pytest.mark.parametrize("N,W,K", [(9001, 1, 13), (9001, 1, 1), (6002, 2, 5), (11000, 4, 3), (11003, 5, 8), (20001, 1, 8)])
+def test_a_sample_does_not_depend_on_the_others(built, N, W, K, tensor_cores):
+    """Past the numbers where the scores, and for few windows the sums, go to kernels of their own: every sample
+    is, to the bit, what it is in a small call (the same operations in the same order), a zero one and one with a NaN
+    among them."""
+    from spi_gb300.sensitivity import fisher
+    gen = torch.Generator(device="cuda").manual_seed(N + W + K)
+    J = torch.randn((N, W, 37, K), device="cuda", generator=gen)
+    J[7] = 0.0
+    J[11, 0, 5, 0] = float("nan")
+    q = torch.rand(37, device="cuda", generator=gen) + 0.1
+    for weight, eps in ((q, 0.0), (None, 1e-6)):
+        whole = fisher(J, weight, eps=eps, tensor_cores=tensor_cores)
+        assert torch.isfinite(whole[1][20:]).all()
+        for rows in (slice(0, 31), slice(N // 2, N // 2 + 2), slice(N - 3, N)):
+            part = fisher(J[rows], weight, eps=eps, tensor_cores=tensor_cores)
+            for a, b in zip(whole, part):
+                assert torch.equal(torch.nan_to_num(a[rows], nan=-7.0), torch.nan_to_num(b, nan=-7.0))
+        assert whole[1][11] == float("-inf") and (eps > 0 or whole[1][7] == float("-inf"))
