@@ -116,10 +116,10 @@ int spi_set_theta(spi_engine* e, const float* theta, int N);
  * mode 1 = weighted squared error with sq_weights[6] (pos, quat, linvel, angvel, q, qd). */
 int spi_set_cost(spi_engine* e, int mode, const float* sq_weights);
 
-/* Rollout-kernel variant: the register allocator targets min_blocks CTAs of 128 threads per
- * SM (2: 255 registers; 3: 168; 4: 128; 5: 96; the quad and block layouts take 3..5, the lane
- * layout 2..4, larger values act as 4). Same equations; results within FP32 rounding of each
- * other. */
+/* Rollout-kernel variant, of a caller's theta batch and of the CEM's population alike: the register
+ * allocator targets min_blocks CTAs of 128 threads per SM (2: 255 registers; 3: 168; 4: 128; 5: 96; the quad and
+ * block layouts take 3..5, the lane layout 2..4, larger values act as 4). Same equations; results within FP32
+ * rounding of each other. */
 int spi_set_kernel_config(spi_engine* e, int min_blocks);
 
 /* Rollout-kernel lane layout (default after spi_create: SPI_LAYOUT_LANE with min_blocks 3).
@@ -135,9 +135,16 @@ int spi_set_kernel_config(spi_engine* e, int min_blocks);
  * barriers per substep; min_blocks 3..5. */
 #define SPI_LAYOUT_BLOCK 2
 int spi_set_kernel_layout(spi_engine* e, int layout);
+/* Layout and variant of one of the two: of a caller's theta batch (population = 0) or of the CEM's population (1). */
+int spi_set_kernel_for(spi_engine* e, int population, int layout, int min_blocks);
 
-/* Roll every (theta, window) pair H control steps and reduce the windowed cost. Async. */
+/* Roll every (theta, window) pair H control steps and reduce the windowed cost. Async. In the lane layout a
+ * caller's theta batch (spi_set_theta) and the CEM's population (spi_cem_init, spi_cem_sample) take kernels of
+ * their own, so the last bits of a cost, though not its accuracy, depend on how the batch was set. */
 int spi_run(spi_engine* e);
+/* spi_run with the population's kernels whoever set the batch: the costs that a CEM iteration or the server gives
+ * these theta samples, to the bit. */
+int spi_run_population(spi_engine* e);
 /* spi_set_theta, spi_run and spi_read_costs in one call: theta device [N][13], comp device [N][9] and
  * cost device [N] (either may be NULL). The same results, without the copies in between. Async. */
 int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* cost);

@@ -30,7 +30,7 @@ int cem_refit_impl(spi_engine* e) {
 
 int cem_step_impl(spi_engine* e) {
   int rc = cem_sample_impl(e);
-  if (!rc) rc = run_impl(e, nullptr);
+  if (!rc) rc = run_impl(e, nullptr, true);
   if (!rc) rc = cem_refit_impl(e);
   return rc;
 }

@@ -60,6 +60,22 @@ int reserve_theta(spi_engine* e, int N) {
   return rc;
 }
 
+int check_kernel(const char* what, int layout, int min_blocks) {
+  if (layout != SPI_LAYOUT_QUAD && layout != SPI_LAYOUT_LANE && layout != SPI_LAYOUT_BLOCK)
+    return set_error(SPI_EINVAL, "%s: layout %d not 0/1/2", what, layout);
+  const int lo = layout == SPI_LAYOUT_LANE ? 2 : 3;
+  if (min_blocks < lo || min_blocks > 5)
+    return set_error(SPI_EINVAL, "%s: min_blocks %d outside [%d, 5]", what, min_blocks, lo);
+  return SPI_OK;
+}
+int prepare_kernel(const char* what, int layout) {
+  if (layout != SPI_LAYOUT_LANE) return SPI_OK;
+  // the parking area is above the 48 KB default for dynamic shared memory
+  cudaError_t ce = items_prepare_lane();
+  if (ce == cudaSuccess) ce = eval_prepare();
+  return ce == cudaSuccess ? SPI_OK : cuda_error(ce, what);
+}
+
 }  // namespace
 
 int spi::reserve_run(spi_engine* e) {
@@ -71,7 +87,7 @@ int spi::reserve_run(spi_engine* e) {
   return rc ? rc : refresh_after_realloc(e);
 }
 
-int spi::run_impl(spi_engine* e, float* trace) {
+int spi::run_impl(spi_engine* e, float* trace, bool population) {
   if (!e) return set_error(SPI_EINVAL, "null engine");
   if (e->W <= 0 || e->H <= 0) return set_error(SPI_ESTATE, "spi_run before spi_load_windows");
   if (e->N <= 0) return set_error(SPI_ESTATE, "spi_run before spi_set_theta");
@@ -82,14 +98,15 @@ int spi::run_impl(spi_engine* e, float* trace) {
   const long long warps = (long long)e->N * G;
   const unsigned grid = blocks_for(warps, 4);
   unsigned long long* bad = (unsigned long long*)e->bad.p;
+  const int layout = e->kernel[population].layout, min_blocks = e->kernel[population].min_blocks;
   if (trace) {
     rollout_kernel<true, 3><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
                                                          e->partial.f(), trace, bad);
-  } else if (e->layout == SPI_LAYOUT_LANE && !e->population) {
+  } else if (layout == SPI_LAYOUT_LANE && !population) {
     const EvalArgs a{win, e->theta.f(), e->partial.f(), e->N, G, bad};
-    const cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);
+    const cudaError_t ce = eval_launch(e->host_model, min_blocks, e->sms, a, e->stream);
     if (ce != cudaSuccess) return cuda_error(ce, "rollout launch");
-  } else if (e->layout != SPI_LAYOUT_BLOCK) {
+  } else if (layout != SPI_LAYOUT_BLOCK) {
     // the server's rollout kernel on a table of one slot (items.h), one warp per work item
     SlotDesc d{};
     d.win = win;
@@ -101,20 +118,20 @@ int spi::run_impl(spi_engine* e, float* trace) {
     d.G = G;
     d.norm = e->norm;
     d.active = 1;
-    const long long items = items_of(e->layout, e->N, G);
+    const long long items = items_of(layout, e->N, G);
     const long long ctas = items_grid(items, 1);
     if (ctas > 0x7fffffffLL) return set_error(SPI_EINVAL, "spi_run: %lld work items", items);
     SingleTable* tab = static_cast<SingleTable*>(e->items.p);
     cudaError_t ce = items_fill_single(tab, d, items, 1, e->stream);
     if (ce == cudaSuccess)
-      ce = items_launch(e->layout, e->min_blocks, e->host_model, e->d_model, single_tables(tab), 0, (int)ctas, bad,
+      ce = items_launch(layout, min_blocks, e->host_model, e->d_model, single_tables(tab), 0, (int)ctas, bad,
                         e->stream);
     if (ce != cudaSuccess) return cuda_error(ce, "rollout launch");
   } else {
-    if (e->min_blocks == 4)
+    if (min_blocks == 4)
       rollout_block_kernel<4><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
                                                             e->partial.f(), bad);
-    else if (e->min_blocks == 5)
+    else if (min_blocks == 5)
       rollout_block_kernel<5><<<grid, 128, 0, e->stream>>>(e->d_model, win, e->theta.f(), e->N, G,
                                                             e->partial.f(), bad);
     else
@@ -225,28 +242,32 @@ int spi_set_theta(spi_engine* e, const float* theta, int N) {
 
 int spi_set_kernel_config(spi_engine* e, int min_blocks) {
   if (!e) return set_error(SPI_EINVAL, "null engine");
-  const int lo = e->layout == SPI_LAYOUT_LANE ? 2 : 3;
-  if (min_blocks < lo || min_blocks > 5)
-    return set_error(SPI_EINVAL, "spi_set_kernel_config: min_blocks %d outside [%d, 5]", min_blocks, lo);
-  e->min_blocks = min_blocks;
+  for (const auto& k : e->kernel)
+    if (int rc = check_kernel("spi_set_kernel_config", k.layout, min_blocks)) return rc;
+  for (auto& k : e->kernel) k.min_blocks = min_blocks;
   if (e->graph_exec) { cudaGraphExecDestroy(e->graph_exec); e->graph_exec = nullptr; }
   return SPI_OK;
 }
 
 int spi_set_kernel_layout(spi_engine* e, int layout) {
   if (!e) return set_error(SPI_EINVAL, "null engine");
-  if (layout != SPI_LAYOUT_QUAD && layout != SPI_LAYOUT_LANE && layout != SPI_LAYOUT_BLOCK)
-    return set_error(SPI_EINVAL, "spi_set_kernel_layout: layout %d not 0/1/2", layout);
-  if (layout == SPI_LAYOUT_LANE) {
-    // the parking area is above the 48 KB default for dynamic shared memory
-    cudaError_t ce = items_prepare_lane();
-    if (ce == cudaSuccess) ce = eval_prepare();
-    if (ce != cudaSuccess) return cuda_error(ce, "spi_set_kernel_layout: shared-memory attribute");
-  } else if (e->min_blocks < 3) {
-    e->min_blocks = 3;
+  int rc = check_kernel("spi_set_kernel_layout", layout, 3);
+  if (rc || (rc = prepare_kernel("spi_set_kernel_layout", layout))) return rc;
+  for (auto& k : e->kernel) {
+    k.layout = layout;
+    if (layout != SPI_LAYOUT_LANE && k.min_blocks < 3) k.min_blocks = 3;
   }
-  e->layout = layout;
   if (e->graph_exec) { cudaGraphExecDestroy(e->graph_exec); e->graph_exec = nullptr; }
+  return SPI_OK;
+}
+
+int spi_set_kernel_for(spi_engine* e, int population, int layout, int min_blocks) {
+  if (!e) return set_error(SPI_EINVAL, "null engine");
+  int rc = check_kernel("spi_set_kernel_for", layout, min_blocks);
+  if (rc || (rc = prepare_kernel("spi_set_kernel_for", layout))) return rc;
+  e->kernel[population != 0].layout = layout;
+  e->kernel[population != 0].min_blocks = min_blocks;
+  if (population && e->graph_exec) { cudaGraphExecDestroy(e->graph_exec); e->graph_exec = nullptr; }
   return SPI_OK;
 }
 
@@ -259,15 +280,17 @@ int spi_set_cost(spi_engine* e, int mode, const float* sq_weights) {
   return SPI_OK;
 }
 
-int spi_run(spi_engine* e) { return run_impl(e, nullptr); }
+int spi_run(spi_engine* e) { return run_impl(e, nullptr, e && e->population); }
+
+int spi_run_population(spi_engine* e) { return run_impl(e, nullptr, true); }
 
 int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* cost) {
   if (!e || !theta) return set_error(SPI_EINVAL, "spi_evaluate: null argument");
   if (N <= 0) return set_error(SPI_EINVAL, "spi_evaluate: N=%d must be > 0", N);
   if (e->W <= 0 || e->H <= 0) return set_error(SPI_ESTATE, "spi_evaluate before spi_load_windows");
-  if (e->layout != SPI_LAYOUT_LANE) {
+  if (e->kernel[0].layout != SPI_LAYOUT_LANE) {
     int rc = spi_set_theta(e, theta, N);
-    if (!rc) rc = run_impl(e, nullptr);
+    if (!rc) rc = run_impl(e, nullptr, false);
     return rc ? rc : spi_read_costs(e, comp, cost);
   }
   const int G = (e->W + 7) / 8;
@@ -283,7 +306,7 @@ int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* c
   }
   const WinView win{e->init.f(), e->act.f(), e->tgt.f(), e->weight.f(), e->W, e->H};
   const EvalArgs a{win, theta, e->partial.f(), N, G, (unsigned long long*)e->bad.p};
-  cudaError_t ce = eval_launch(e->host_model, e->min_blocks, e->sms, a, e->stream);
+  cudaError_t ce = eval_launch(e->host_model, e->kernel[0].min_blocks, e->sms, a, e->stream);
   if (ce != cudaSuccess) return cuda_error(ce, "spi_evaluate: rollout launch");
   const float* w = e->sq_w;
   finalize_evaluate<<<blocks_for(N, 128), 128, 0, e->stream>>>(e->partial.f(), N, G, e->norm, e->cost_mode, w[0], w[1],
@@ -297,7 +320,7 @@ int spi_evaluate(spi_engine* e, const float* theta, int N, float* comp, float* c
 
 int spi_run_trace(spi_engine* e, float* trace) {
   if (!trace) return set_error(SPI_EINVAL, "spi_run_trace: null trace");
-  return run_impl(e, trace);
+  return run_impl(e, trace, false);
 }
 
 int spi_read_costs(spi_engine* e, float* comp, float* cost) {

@@ -23,8 +23,8 @@ struct spi_engine {
   int cost_mode = 1;
   float sq_w[6] = {10.f, 5.f, 0.1f, 0.1f, 1.f, 0.01f};
   bool ran = false;
-  int min_blocks = 3;                      // rollout kernel occupancy variant
-  int layout = 0;                          // SPI_LAYOUT_QUAD / SPI_LAYOUT_LANE
+  // rollout kernel of a caller's theta batch and of the CEM's population: lane layout, occupancy variant
+  struct { int layout = 0, min_blocks = 3; } kernel[2];
   spi::DeviceBuf items;                    // one-slot work table of the rollout kernel (items.h)
   // CEM
   spi::DeviceBuf cem;                      // one CemState
@@ -39,7 +39,8 @@ struct spi_engine {
 };
 
 namespace spi {
-int run_impl(spi_engine* e, float* trace);
+// population: with the kernels of the CEM's population (trace: neither's)
+int run_impl(spi_engine* e, float* trace, bool population);
 // The buffers of a run over the engine's theta batch; what depends on their addresses follows them.
 int reserve_run(spi_engine* e);
 // Call after any DeviceBuf::reserve of theta / cost / partial / comp / windows: if one of

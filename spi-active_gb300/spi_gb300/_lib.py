@@ -37,6 +37,8 @@ ENGINE_API = {
     "spi_set_cost": (c_int, [c_void_p, c_int, POINTER(c_float)]),
     "spi_run": (c_int, [c_void_p]),
     "spi_evaluate": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+    "spi_run_population": (c_int, [c_void_p]),
+    "spi_set_kernel_for": (c_int, [c_void_p, c_int, c_int, c_int]),
     "spi_set_kernel_config": (c_int, [c_void_p, c_int]),
     "spi_set_kernel_layout": (c_int, [c_void_p, c_int]),
     "spi_run_trace": (c_int, [c_void_p, c_void_p]),

@@ -69,13 +69,17 @@ class CEM:
         self.cfg = c
         self.lo, self.hi = lo, hi
         _lib.check(self.lib.spi_cem_init(engine._h, ctypes.byref(c)))
-        engine.N = int(n_samples)
+        self._take_batch()
+
+    def _take_batch(self):
+        """The engine's theta batch is this population (again)."""
+        self.engine.N, self.engine.population = self.cfg.n_samples, True
 
     def step(self, rollout_events=None):
         """One iteration: sample, roll every (theta, window), refit. Events bracket the rollout."""
         h = self.engine._h
         _lib.check(self.lib.spi_cem_sample(h))
-        self.engine.N = self.cfg.n_samples   # the engine's batch is the population
+        self._take_batch()
         if rollout_events:
             rollout_events[0].record(self.engine.stream)
         _lib.check(self.engine.lib.spi_run(h))
@@ -85,7 +89,7 @@ class CEM:
 
     def sample(self):
         _lib.check(self.lib.spi_cem_sample(self.engine._h))
-        self.engine.N = self.cfg.n_samples
+        self._take_batch()
 
     def refit(self):
         _lib.check(self.lib.spi_cem_refit(self.engine._h))
@@ -93,7 +97,7 @@ class CEM:
     def run(self, iterations, graph=True):
         _lib.check(self.lib.spi_cem_run(self.engine._h, int(iterations), int(bool(graph))))
         if iterations:
-            self.engine.N = self.cfg.n_samples
+            self._take_batch()
 
     def read(self):
         P = len(self.param_ids)

@@ -51,6 +51,7 @@ class Engine:
         self.stream = stream or torch.cuda.current_stream(self.device)
         _lib.check(self.lib.spi_set_stream(self._h, ctypes.c_void_p(self.stream.cuda_stream)))
         self.W = self.H = self.N = 0
+        self.population = False    # the theta batch is a CEM's population
         self._keep = []
         if variant is not None:
             from .autotune import set_variant
@@ -90,17 +91,20 @@ class Engine:
         _lib.check(self.lib.spi_set_theta(self._h, theta.data_ptr(), theta.shape[0]))
         self._theta = theta
         self.N = theta.shape[0]
+        self.population = False
 
     def set_cost(self, mode=COST_SQ, sq_weights=DEFAULT_SQ_WEIGHTS):
         w = (ctypes.c_float * 6)(*sq_weights)
         _lib.check(self.lib.spi_set_cost(self._h, int(mode), w))
 
-    def run(self, trace=False):
+    def run(self, trace=False, population=False):
+        """Roll the theta batch. population: with the kernels that a CEM's population takes, for that CEM's
+        costs to the bit."""
         if trace:
             tr = torch.empty((self.N, self.W, self.H, STATE_DIM), device=self.device, dtype=torch.float32)
             _lib.check(self.lib.spi_run_trace(self._h, tr.data_ptr()))
             return tr
-        _lib.check(self.lib.spi_run(self._h))
+        _lib.check((self.lib.spi_run_population if population else self.lib.spi_run)(self._h))
         return None
 
     def read(self, out_comp=None, out_cost=None):
@@ -129,6 +133,7 @@ class Engine:
         if rc not in (_lib.SPI_EINVAL, _lib.SPI_ESTATE):   # the batch is set, also where the run found no memory
             self._theta = theta
             self.N = N
+            self.population = False
         _lib.check(rc)
         return comp, cost
 

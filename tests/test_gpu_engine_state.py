@@ -93,3 +93,41 @@ def test_cem_after_an_evaluation_without_memory(built):
         got.append((cem.theta(), e.read()[1], cem.read()["best_cost"]))
         e.close()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2]
+
+
+@pytest.mark.parametrize("variant", ["lane2", "lane3", "quad4"])
+def test_a_callers_batch_by_the_populations_kernels(built, variant):
+    """The CEM's theta samples set by the caller and run as a population: the CEM's costs, to the bit; its own choice of
+    kernel leaves the other's alone."""
+    from spi_gb300 import _lib
+    from spi_gb300.autotune import _BY_NAME, set_variant
+    windows = _windows(19)
+    e, other = _engine(windows), _engine(windows)
+    set_variant(e, "lane3")
+    _, layout, min_blocks = _BY_NAME[variant]
+    for x in (e, other):
+        _lib.check(x.lib.spi_set_kernel_for(x._h, 1, layout, min_blocks))
+    cem = _cem(e)
+    cem.sample()
+    th = cem.theta()
+    e.run()
+    comp, cost = e.read()
+    other.set_theta(th)
+    other.run(population=True)
+    c, v = other.read()
+    assert torch.equal(c, comp) and torch.equal(v, cost)
+    plain = _engine(windows).evaluate(th)[1]
+    assert torch.equal(other.evaluate(th)[1], plain)
+
+
+def test_tuning_keeps_a_choice_for_each_batch(built, monkeypatch, tmp_path):
+    from spi_gb300 import autotune
+    monkeypatch.setattr(autotune, "CACHE", tmp_path / "autotune.json")
+    e = _engine(_windows(19))
+    e.evaluate(torch.from_numpy(random_theta(np.random.default_rng(4), 64).astype(np.float32)))
+    best, ms = autotune.tune_engine(e)
+    assert best in ms and set(ms) == {v[0] for v in autotune.VARIANTS}
+    cem = _cem(e)
+    cem.run(2)
+    assert np.isfinite(cem.read()["best_cost"])
+    assert autotune.tune_engine(e)[0] in ms
