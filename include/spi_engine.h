@@ -126,8 +126,9 @@ int spi_set_kernel_config(spi_engine* e, int min_blocks);
  * SPI_LAYOUT_QUAD: four lanes per rollout, one leg each, the base
  * solved on all four. SPI_LAYOUT_LANE: one lane per rollout through all four legs, the model
  * in the kernel's parameter block, 68 KB of shared memory per 128-thread CTA (three CTAs per
- * SM); min_blocks 2..4 sets the register cap (4: 128 registers). Same equations, results
- * within FP32 rounding of each other; spi_run_trace always uses the quad layout. */
+ * SM); min_blocks 2..4 sets the register cap (4: 128 registers; on a caller's theta batch 4 acts as
+ * 3). Same equations, results within FP32 rounding of each other; spi_run_trace always uses the
+ * quad layout. */
 #define SPI_LAYOUT_QUAD 0
 #define SPI_LAYOUT_LANE 1
 /* SPI_LAYOUT_BLOCK: the quad layout with each rollout's base solved once per substep by one

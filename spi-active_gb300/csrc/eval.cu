@@ -130,18 +130,19 @@ bool use_team(long long pairs, int sms) {
   return team <= 3 || (lane == 2 && team <= 6);
 }
 
+// The register cap that min_blocks asks for, up to three CTAs per SM: more do not fit beside their 72 KB of shared
+// memory, and the cap of four (128 registers) costs the 148-register kernel 48 bytes of spills for nothing
+// (2048 theta x 64 windows x H = 20: 1,059 us at three, 1,092 under that cap).
 const void* lane_kernel(int min_blocks, bool sl) {
   if (min_blocks <= 2)
     return sl ? (const void*)eval_lane_kernel<2, kMotorSpeedLimit> : (const void*)eval_lane_kernel<2, kMotorRuntime>;
-  if (min_blocks == 3)
-    return sl ? (const void*)eval_lane_kernel<3, kMotorSpeedLimit> : (const void*)eval_lane_kernel<3, kMotorRuntime>;
-  return sl ? (const void*)eval_lane_kernel<4, kMotorSpeedLimit> : (const void*)eval_lane_kernel<4, kMotorRuntime>;
+  return sl ? (const void*)eval_lane_kernel<3, kMotorSpeedLimit> : (const void*)eval_lane_kernel<3, kMotorRuntime>;
 }
 
 }  // namespace
 
 cudaError_t eval_prepare() {
-  for (int mb = 2; mb <= 4; ++mb)
+  for (int mb = 2; mb <= 3; ++mb)
     for (bool sl : {false, true}) {
       const cudaError_t ce =
           cudaFuncSetAttribute(lane_kernel(mb, sl), cudaFuncAttributeMaxDynamicSharedMemorySize, kHipSlotBytes);

@@ -18,7 +18,8 @@ struct EvalArgs {
 
 // Raise the dynamic shared-memory limit of the lane-form kernels.
 cudaError_t eval_prepare();
-// Launch the rollouts of `a` on a GPU of `sms` SMs. min_blocks 2..4: the lane form's register cap.
+// Launch the rollouts of `a` on a GPU of `sms` SMs. min_blocks: the lane form's register cap (2: 255
+// registers, 3 and more: 168).
 cudaError_t eval_launch(const EvalModel& model, int min_blocks, int sms, const EvalArgs& a, cudaStream_t stream);
 
 }  // namespace spi
