@@ -343,19 +343,18 @@ def run_c3(args):
             times.append(time.perf_counter() - t0)
             parts.append(tm)
     breakdown = {k: float(np.mean([p[k] for p in parts])) for k in parts[0]}
-    # the sensitivity kernel against the FP32 peak: FP operations of the dual-number rollout (the
-    # kernel's formulation, one tangent, phase B once) per tangent rollout-step
+    # the sensitivity kernels against the FP32 peak, by the FP operations that they carry out
     from spi_gb300.engine import probe_fp32_peak
-    from spi_gb300.flops import dual_flops_per_rollout_step
-    dual_fl = dual_flops_per_rollout_step(cfg)
+    from spi_gb300.flops import sensitivity_flops_per_rollout_step
+    sens_fl = sensitivity_flops_per_rollout_step(cfg, 13)
     sens_roof = {"kernel": "sensitivity_kernel, tangent_kernel", "bound": "fp32",
-                 "achieved": n * wpc * H * 13 * dual_fl / (breakdown["sensitivities_ms"] * 1e-3) / 1e12,
+                 "achieved": n * wpc * H * sens_fl / (breakdown["sensitivities_ms"] * 1e-3) / 1e12,
                  "peak": probe_fp32_peak() / 1e12, "unit": "TFLOP/s",
-                 "flops_per_tangent_rollout_step": dual_fl,
-                 "note": "achieved = tangent rollout-steps x FP operations of one dual-number control step "
-                         "(csrc/dual.cuh arithmetic, counted on the host; phase B once) / the sensitivity "
-                         "phase's device time; the directions past the first take fewer operations "
-                         "(csrc/tangent.cuh), so this is the rate of the dual-number work replaced; peak: the FP32 FMA-loop probe of this GPU"}
+                 "flops_per_rollout_step": sens_fl,
+                 "note": "achieved = rollout-steps x FP operations of one control step's 13 directions, as carried "
+                         "out and counted on the host (one on the dual scalar, csrc/dual.cuh; twelve tangents and "
+                         "their shared tape, csrc/tangent.cuh; quad-redundant base work once) / the sensitivity "
+                         "phase's device time; peak: the FP32 FMA-loop probe of this GPU"}
     sens_roof["frac"] = sens_roof["achieved"] / sens_roof["peak"]
     # the Fisher reduction alone, tensor cores against CUDA cores, on the last Jacobians
     J, q = r["J"], block_weights((10.0, 5.0, 0.1, 0.1, 1.0, 0.01))
@@ -676,39 +675,36 @@ def run_ours(args):
     steps_per_iter = N * W * H
     value, total_ms = ranks.whole_job_rate(steps_per_iter * args.steps, float(np.sum(step_ms)), dev)
 
-    # end to end: host buffers through the public API, copies inside the timed region
+    # end to end: the same CEM iteration through the public API, its windows from host memory and its costs back
+    # inside the timed region
     e2e = None
     if not args.no_e2e:
         pin = lambda a: torch.from_numpy(np.ascontiguousarray(a)).pin_memory()   # noqa: E731
         h_init, h_act, h_tgt = pin(init), pin(actions), pin(target)
-        h_theta = pin(cem.sample_host(args.steps))
         h_cost = torch.empty((N,), dtype=torch.float32).pin_memory()
         d_init = torch.empty_like(h_init, device=dev)
         d_act = torch.empty_like(h_act, device=dev)
         d_tgt = torch.empty_like(h_tgt, device=dev)
-        d_theta = torch.empty((N, 13), device=dev)
         torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(stream)
-        for k in range(args.steps):
+        for _ in range(args.steps):
             d_init.copy_(h_init, non_blocking=True)
             d_act.copy_(h_act, non_blocking=True)
             d_tgt.copy_(h_tgt, non_blocking=True)
-            d_theta.copy_(h_theta[k], non_blocking=True)
             eng.load_windows(d_init, d_act, d_tgt)
-            eng.set_theta(d_theta)
-            eng.run()
+            cem.step()
             _, cost = eng.read()
             h_cost.copy_(cost, non_blocking=True)
         e1.record(stream)
         torch.cuda.synchronize()
         ranks.barrier()
         e2e_value, e2e_ms = ranks.whole_job_rate(steps_per_iter * args.steps, e0.elapsed_time(e1), dev)
-        h2d = (init.nbytes + actions.nbytes + target.nbytes + N * 13 * 4)
+        h2d = init.nbytes + actions.nbytes + target.nbytes
         e2e = {"value": e2e_value, "unit": METRIC,
                "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(N * 4),
-               "note": "per step: windows + theta H2D from pinned memory, spi_load_windows, "
-                       "spi_set_theta, spi_run, spi_read_costs, cost D2H (evaluation only)"}
+               "note": "per step: windows H2D from pinned memory, spi_load_windows, one CEM iteration (sample, "
+                       "rollouts, refit; the population is drawn on the device), spi_read_costs, cost D2H"}
 
     fl = flops_per_rollout_step(cfg)
     kmean = float(np.mean(kern_ms))

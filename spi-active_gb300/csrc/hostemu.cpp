@@ -40,6 +40,8 @@ inline Cf& operator-=(Cf& a, Cf b) { a = a - b; return a; }
 inline bool operator>(Cf a, Cf b) { return a.v > b.v; }
 inline bool operator<=(Cf a, Cf b) { return a.v <= b.v; }
 inline bool operator<(Cf a, Cf b) { return a.v < b.v; }
+inline bool operator>=(Cf a, Cf b) { return a.v >= b.v; }
+inline bool operator==(Cf a, Cf b) { return a.v == b.v; }
 inline Cf m_sqrt(Cf x) { ++Cf::n; return Cf(std::sqrt(x.v)); }
 inline Cf m_tanh(Cf x) { ++Cf::n; return Cf(std::tanh(x.v)); }
 inline void m_sincos(Cf x, Cf* s, Cf* c) { Cf::n += 2; *s = Cf(std::sin(x.v)); *c = Cf(std::cos(x.v)); }
@@ -602,6 +604,65 @@ int spi_hostemu_count_ops_dual(const spi_robot* robot, const double* state, cons
   Cf::n = 0;
   substep<false>(M, B, L, bp, lp, act);
   *per_substep = Cf::n;
+  return SPI_OK;
+}
+
+// FP operations of one substep of one direction by tangents (tangent.cuh) and of the tape that a pair's directions
+// may share (the residual with its intermediates); the solve with the kept 6x6 factor is counted by hand.
+int spi_hostemu_count_ops_tangent(const spi_robot* robot, const double* state, const double* theta, const double* act12,
+                                  long long* per_direction, long long* tape) {
+  DevModel M;
+  const char* why = "";
+  int rc = build_dev_model(*robot, &M, &why);
+  if (rc) return rc;
+  BaseState<Cf> B;
+  LegState<Cf> L[4];
+  BaseParams<Cf> bp;
+  LegParams<Cf> lp[4];
+  load_rollout(M, state, theta, B, L, bp, lp);
+  Cf tgt[12];
+  for (int j = 0; j < 12; ++j) tgt[j] = joint_target(M, j % 3, j / 3, Cf(act12[j]));
+  adj::SolveWork<Cf> W[4];
+  LegOut<Cf> sum = base_terms(bp, B);
+  for (int leg = 0; leg < 4; ++leg) phase_a_into(M, leg, B, L[leg], lp[leg], tgt + 3 * leg, W[leg], sum, false);
+  const BaseState<Cf> B0 = B;
+  const SV<Cf> a0 = base_solve(M, sum.I, sum.p, B);
+  adj::LegTape<Cf> t[4];
+  Cf qdd[4][3];
+  Cf::n = 0;
+  for (int leg = 0; leg < 4; ++leg) {
+    Cf r[3];
+    SV<Cf> fb;
+    adj::leg_qdd(W[leg], a0, qdd[leg]);
+    adj::leg_pose(B0, L[leg], t[leg]);
+    adj::leg_residual<kMotorRuntime>(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, a0, qdd[leg], t[leg], r, fb);
+  }
+  *tape = Cf::n;
+  tng::BaseTan<Cf> dB = tng::zero_base_tan<Cf>();
+  tng::ParamTan<Cf> dP = {};
+  Cf::n = 0;
+  SV<Cf> x = tng::base_residual_tan(bp, B0, a0, dB, dP);
+  Cf z[4][3];
+  tng::LegTan<Cf> dL[4] = {};
+  for (int leg = 0; leg < 4; ++leg) {
+    Cf dr[3];
+    SV<Cf> dfb;
+    tng::leg_residual_tan(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, qdd[leg], t[leg], t[leg].zf, {true, false}, dB, dL[leg], dP, dr,
+                          dfb);
+    adj::add_sv(x, dfb);
+    adj::add_sv(x, adj::leg_solve_down(W[leg], dr, z[leg]));
+  }
+  Cf::n += 72;                                     // 2 (15 multiplies and subtractions, 6 multiplies)
+  tng::base_integrate_tan(M, B0, B, a0, dB);
+  for (int leg = 0; leg < 4; ++leg) {
+    Cf dqdd[3];
+    adj::leg_solve_up(W[leg], z[leg], a0, dqdd);
+    for (int i = 0; i < 3; ++i) {
+      dL[leg].qd[i] = dL[leg].qd[i] + Cf(M.dt) * dqdd[i];
+      dL[leg].q[i] = dL[leg].q[i] + Cf(M.dt) * dL[leg].qd[i];
+    }
+  }
+  *per_direction = Cf::n;
   return SPI_OK;
 }
 
