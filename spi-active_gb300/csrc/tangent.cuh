@@ -82,18 +82,13 @@ SPI_INL V3<T> contact_tan(const DevModel& M, T radius, T z, V3<T> v, V3<T> n, Co
   dmimp = dmds * ds;
   const T dfz = dfn + dmimp * T(M.g);
   // The branch is the forward pass's, vt is formed here, with other roundings: a slip's speed may come out as zero.
-  // Off, a slip has no friction whatever its speed; on, the value at rest is the sticking one.
-  T scale = T(M.ct), dscale = T(0);
-  if (!br.stick) {
-    const T vv = dot(vt, vt);
-    if (!br.on) {
-      scale = T(0);
-    } else if (vv > T(0)) {
-      const T inv = T(1) / m_sqrt(vv);
-      scale = T(M.mu) * fn * inv;
-      dscale = (T(M.mu) * dfn - scale * dot(vt, dvt) * inv) * inv;
-    }
-  }
+  // Off, a slip has no friction whatever its speed; on, the value at rest is the sticking one. (Selected, not branched
+  // on: 4096 windows x 13 directions 1.53 ms, 1.57 with a branch.)
+  const T vv = dot(vt, vt);
+  const bool slides = br.on && !br.stick && vv > T(0);
+  const T inv = T(1) / m_sqrt(vv);
+  const T ss = T(M.mu) * fn * inv, dss = (T(M.mu) * dfn - ss * dot(vt, dvt) * inv) * inv;
+  const T scale = slides ? ss : (br.stick || br.on ? T(M.ct) : T(0)), dscale = slides ? dss : T(0);
   return v3(dfz * n.x + fz * dn.x - dscale * vt.x - scale * dvt.x, dfz * n.y + fz * dn.y - dscale * vt.y - scale * dvt.y,
             dfz * n.z + fz * dn.z - dscale * vt.z - scale * dvt.z);
 }
