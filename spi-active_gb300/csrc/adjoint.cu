@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128) adjoint_forward_kernel(const DevModel* __
 
 // Bound by its arithmetic at the 8 warps per SM that 255 registers leave (62 % of the issue slots). As one kernel
 // with the forward pass, each substep computed again from its state, it waited for instructions 2.5
-// cycles an issue: 14.3 ms for 512 theta x 256 windows x H = 20, 7.26 ms as two. The kept fields come
+// cycles an issue: 13.4 ms for 512 theta x 256 windows x H = 20, 6.15 ms as two. The kept fields come
 // straight from memory; staged a substep ahead in shared memory they took the same time.
 __global__ void __launch_bounds__(128) adjoint_reverse_kernel(const DevModel* __restrict__ model, const AdjArgs a) {
   __shared__ DevModel M;

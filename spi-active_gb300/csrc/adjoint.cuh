@@ -234,7 +234,9 @@ template <class T> struct LegTape {
 
 // a b + c d, c d rounded first. The contacts' branches (on or off, stick or slip) turn on the last bits of the
 // foot's height and velocity: left to the compiler, which product of a rotation is fused varies with the code
-// around it, and with it the branch, hence the gradient, of the few contacts at an edge.
+// around it, and with it the branch, hence the gradient, of the few contacts at an edge. This fixes the rotations, where
+// two builds were seen to part; the height's sums and the foot's linear velocity are still the compiler's, so
+// that a contact within a rounding of an edge may be taken on the side that the trajectory did not take.
 template <class T> SPI_INL T mul_add2(T a, T b, T c, T d) { return a * b + c * d; }
 #ifdef __CUDA_ARCH__
 template <> SPI_INL float mul_add2<float>(float a, float b, float c, float d) {

@@ -78,8 +78,9 @@ __global__ void __launch_bounds__(128, MINB) eval_lane_kernel(const __grid_const
   window_result(a.win, w, active, s13, L, live ? a.partial + (size_t)q * SPI_N_COMP : nullptr, a.n_bad);
 }
 
-// Latency-bound: one chain of substeps per rollout, at most a few warps per scheduler. 64 theta x 8 windows
-// x H = 5: 26 us for the launch and its finalize, against 57 us with one lane per rollout.
+// Latency-bound: one chain of substeps per rollout, at most a few warps per scheduler (0.43 of the issue slots of an SM
+// with one CTA). 64 theta x 8 windows x H = 5: 26 us for the launch and its finalize, against 57 us with
+// one lane per rollout.
 template <int MS>
 __global__ void __launch_bounds__(128) eval_team_kernel(const __grid_constant__ EvalModel M, const EvalArgs a) {
   __shared__ TeamShare share_cta[4];

@@ -8,8 +8,9 @@
 //   lane layout  four consecutive (theta, eight-window group) items of one slot, one lane per
 //                window (rollout_lane_item).
 // Results go to the slot's partial[(n G + g)][SPI_N_COMP]; where an item runs does not change
-// them. This is the only translation unit that instantiates the rollout for spi_run, the engine
-// CEM and spi_server_tick, so the three produce bitwise-identical partials for the same job.
+// them. This is the only translation unit that instantiates the rollout for the engine CEM, spi_run_population
+// and spi_server_tick (and for spi_run in the quad layout), so these produce bitwise-identical partials for
+// the same job. In the lane layout spi_run on a caller's theta batch takes eval.cu.
 #include <cuda_runtime.h>
 
 #include "items.h"

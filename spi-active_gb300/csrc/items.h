@@ -3,8 +3,8 @@
 // Both the engine CEM (and spi_run in the quad layout) and the continuous-batching server
 // (spi_server_tick) evaluate their (theta, window) pairs with the same kernels, defined once in
 // items.cu: every warp takes a work item and looks up, in a slot table, which job the item belongs
-// to. The engine is a table of one slot. (spi_run in the lane layout on a population that the CEM did
-// not draw, and spi_evaluate, take the kernels of eval.cu.) Because both callers launch
+// to. The engine is a table of one slot. (In the lane layout spi_run on a theta batch of the caller's and
+// spi_evaluate take the kernels of eval.cu; spi_run_population takes these on any batch.) Because both callers launch
 // the same compiled kernel, a job's costs are bitwise identical whether it runs alone on the
 // engine or inside the server's mix; two separately compiled copies of the rollout may contract
 // different multiply-add pairs into FMAs and differ in the last bit.

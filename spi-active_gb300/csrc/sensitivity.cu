@@ -6,7 +6,8 @@
 //     one lane quad per (sample, window, direction). Each direction carries the whole trajectory, the
 //     legs' condensation and the Cholesky factorisation along: some 4,000 instructions a substep;
 //   * the first direction that way, keeping each substep's solve, and the others by tangent.cuh from
-//     the kept substeps, one quad per (sample, window, direction) too, a quarter of the instructions.
+//     the kept substeps, one quad per (sample, window, direction) too, 0.46 of the instructions (0.40
+//     where a pair's directions share a tape).
 // The second runs two chains one after the other, so it takes over where the dual rollouts no longer
 // fit the GPU at once (use_tangents).
 // With K <= 13 parameters and a 37-dimensional state, K forward tangents give the whole
@@ -240,9 +241,10 @@ __device__ __forceinline__ void load_tape(const float4* d, adj::LegTape<float>& 
 
 // Directions 1 .. K - 1 from the kept substeps, one lane quad per (pair, direction), a pair's directions side by
 // side. Bound by its arithmetic at the 8 or 12 warps per SM that its registers leave (0.67, 0.63 instructions a
-// cycle; with TAPES the warps wait for the one that forms the next tape). The CTA's pairs (three or four for K = 13) have their kept substeps staged through shared memory by
-// asynchronous copies two substeps ahead, three buffers in turn; read straight from memory, two warps per
-// scheduler waited for each substep's loads twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
+// cycle; with TAPES the warps wait for the one that forms the next tape). The CTA's pairs (three or four for
+// K = 13) have their kept substeps staged through shared memory by asynchronous copies two substeps ahead,
+// three buffers in turn; read straight from memory, two warps per scheduler waited for each substep's loads
+// twice (1.5 ms at 4096 pairs x 12 directions x H = 20; 1.2 ms so).
 //
 // TAPES: the part of the residual that a pair's directions share (sines, velocities, accelerations, forces: a
 // third of a direction's instructions) is formed once per pair, a substep ahead, one lane per leg, the
@@ -405,9 +407,11 @@ constexpr size_t kScratch = (size_t)4 << 30;   // bytes of kept substeps
 // take more than `waves` times the warps that fit the GPU at once (two CTAs of 255 registers a thread per
 // SM). The first direction's chain comes before the others', so below two waves the dual rollouts are done
 // first, and with two directions it does not come back (H = 20, 152 SMs, dual against tangents):
-//   1100 pairs x 13   0.77 / 0.92 ms      1530 x 13   1.13 / 0.93 ms      4096 x 13   2.30 / 1.55 ms
-//   4900 pairs x 3    0.79 / 0.95 ms      6600 x 3    1.13 / 1.03 ms     10000 x 2    1.13 / 1.35 ms
-// Batches follow one another, each with a last wave of its own; several of them need twice as much each.
+//   1100 pairs x 13   0.80 / 0.85 ms      1530 x 13   1.16 / 0.86 ms      4096 x 13   2.33 / 1.55 ms
+//   4900 pairs x 3    0.79 / 0.96 ms      6600 x 3    1.15 / 1.03 ms     10000 x 2    1.13 / 1.35 ms
+// Batches follow one another, each with a last wave of its own, so that several of them ask for more each. Five
+// batches at 2.2, 3.0 and 3.7 waves: H = 200, K = 3, 4, 5: 45.8 / 50.5, 60.2 / 60.1, 74.2 / 58.0 ms; H = 400, K = 6, 8,
+// 10: 91.9 / 92.4, 121 / 112, 149 / 131. Four waves, at which none of them loses.
 constexpr int kDualWaves = 2;
 bool use_tangents(long long pairs, int K, int sms, int waves) {
   return K >= 3 && pairs * K > (long long)waves * 2 * 32 * sms;
@@ -421,8 +425,8 @@ int tangent_smem(int K, bool tapes) {
 
 // Whether the tangents of a pair share one tape: with four or more to share it, and over two waves of the two
 // CTAs per SM that fit otherwise (H = 20, 152 SMs, whole call, own tapes against shared ones):
-//   4096 pairs x 13   1.69 / 1.55 ms      1650 x 13   1.06 / 1.00 ms      1530 x 13   0.86 / 0.92 ms
-//   8192 pairs x 5    1.43 / 1.40 ms      8192 x 4    1.25 / 1.34 ms
+//   4096 pairs x 13   1.67 / 1.55 ms      1650 x 13   0.98 / 0.94 ms      1530 x 13   0.86 / 0.94 ms
+//   8192 pairs x 5    1.40 / 1.40 ms      8192 x 4    1.23 / 1.28 ms      4096 x 5    0.96 / 1.05 ms
 bool use_tapes(long long pairs, int K, int sms) {
   return K >= 5 && pairs * (K - 1) > (long long)2 * 2 * 32 * sms;
 }
