@@ -13,7 +13,7 @@
 //      order) into one partial per (theta, window group); adjoint_finalize sums a theta's partials
 //      in group order and divides by the window normaliser, as the cost of spi_run does.
 // The kept substeps are 736 bytes each per rollout, written and read once in 16-byte fields, a warp's
-// accesses contiguous. They take kScratch at most: (theta, group) pairs go through in batches, and a
+// accesses contiguous. They take 4 GB at most (ScratchLimit): (theta, group) pairs go through in batches, and a
 // horizon over kSegSteps control steps in segments from checkpoints of the state (the segments'
 // forward passes run again, last segment first, the adjoint carried in memory).
 #include <cuda_runtime.h>
@@ -30,7 +30,6 @@ using namespace spi;
 namespace {
 
 constexpr int kSegSteps = 50;                       // control steps between checkpoints
-constexpr size_t kScratch = (size_t)4 << 30;        // bytes of kept substeps
 constexpr size_t kPairBytes = 8 * kKeptBytes;       // a warp's eight rollouts', per substep
 
 // Phase A's work record to its parking slot (for phase C) and to the kept substep.
@@ -427,16 +426,18 @@ extern "C" int spi_adjoint(spi_engine* e, const float* theta, int N, float* cost
   const long long all = (long long)N * G;
   const int seg = std::min(H, kSegSteps), bounds = (H - 1) / kSegSteps;   // boundaries inside the horizon
   const size_t slots = (size_t)seg * dec + 1;
-  // batches of equal size within kScratch; smaller ones when the device has less to give
-  const long long most = std::max(1LL, (long long)(kScratch / (slots * kPairBytes)));
-  long long batches = (all + most - 1) / most, batch;
+  // batches of equal size within the engine's limit; smaller ones when the device has less to give
+  long long batch;
   int rc;
-  for (;; batches *= 2) {
+  for (e->adj_limit.begin_call();; e->adj_limit.refused(slots * batch * kPairBytes)) {
+    const long long most = std::max(1LL, (long long)(e->adj_limit.bytes / (slots * kPairBytes)));
+    const long long batches = (all + most - 1) / most;
     batch = (all + batches - 1) / batches;
     rc = e->adj_seg.reserve(slots * batch * kPairBytes);
     if (!rc) rc = e->adj_ckpt.reserve(bounds * batch * (kPairBytes + (size_t)32 * 32 * sizeof(float)));
     if (rc != SPI_ENOMEM || batch == 1) break;
   }
+  if (rc == SPI_ENOMEM) e->adj_limit = ScratchLimit();   // nothing to be had: the next call begins anew
   if (!rc) rc = e->adj_part.reserve((size_t)all * (SPI_THETA_DIM + 1) * sizeof(float));
   if (rc) return rc;
   AdjArgs a;

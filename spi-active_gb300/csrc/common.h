@@ -38,4 +38,17 @@ struct DeviceBuf {
   double* d() const { return static_cast<double*>(p); }
 };
 
+// How much scratch an engine asks the device for: 4 GB at first, half of what was refused from then on, and 256 calls later
+// all of it again, since memory may have come free. A refused allocation takes 0.25 ms and one that goes and
+// comes back on each call 8 ms, so a call does not ask for what the last one did not get.
+struct ScratchLimit {
+  static constexpr size_t kMost = (size_t)4 << 30;
+  size_t bytes = kMost;
+  int calls = 0;
+  void begin_call() {
+    if (bytes < kMost && ++calls >= 256) *this = ScratchLimit();
+  }
+  void refused(size_t asked) { bytes = asked / 2; }
+};
+
 }  // namespace spi

@@ -34,8 +34,10 @@ struct spi_engine {
   cudaStream_t capture_stream = nullptr;   // graphs are captured here, replayed on `stream`
   unsigned seen_generation = 0;            // buffer generations the graph / CEM pointers refer to
   spi::DeviceBuf sens_kept;                // kept substeps of the sensitivities' first direction
+  spi::ScratchLimit sens_limit;
   cudaEvent_t sens_done = nullptr;         // after the last call that used sens_kept
   spi::DeviceBuf adj_ckpt, adj_seg, adj_part;   // adjoint checkpoints, kept substeps, partials
+  spi::ScratchLimit adj_limit;             // of adj_seg
 };
 
 namespace spi {

@@ -401,8 +401,6 @@ __global__ void __launch_bounds__(128, TAPES ? 3 : 2) tangent_kernel(const DevMo
   }
 }
 
-constexpr size_t kScratch = (size_t)4 << 30;   // bytes of kept substeps
-
 // Whether the directions past the first go by tangents: three directions or more whose dual rollouts would
 // take more than `waves` times the warps that fit the GPU at once (two CTAs of 255 registers a thread per
 // SM). The first direction's chain comes before the others', so below two waves the dual rollouts are done
@@ -727,16 +725,22 @@ int spi_sensitivity(spi_engine* e, const float* theta, int N, const int32_t* par
   a.xH = xH;
   const long long all = (long long)N * e->W;
   const size_t slots = (size_t)e->H * e->host_model.decimation + 1;
-  // batches of equal size within kScratch. A capture keeps to the dual rollouts, which need no memory of the
-  // engine's: a graph would go on using what a later call may replace.
-  const long long most = std::max(1LL, (long long)(kScratch / (slots * kKeptBytes)));
-  const long long batches = (all + most - 1) / most;
-  long long batch = (all + batches - 1) / batches;
+  // Batches of equal size within the engine's limit. A capture keeps to the dual rollouts, which need no memory of
+  // the engine's: a graph would go on using what a later call may replace.
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  const bool split = use_tangents(batch, K, e->sms, batches > 1 ? 2 * kDualWaves : kDualWaves) &&
-                     cudaStreamIsCapturing(e->stream, &capture) == cudaSuccess &&
-                     capture == cudaStreamCaptureStatusNone &&
-                     e->sens_kept.reserve(slots * batch * kKeptBytes) == SPI_OK;
+  const bool may = cudaStreamIsCapturing(e->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+  long long batch = all;
+  bool split = false;
+  e->sens_limit.begin_call();
+  while (may && !split) {
+    const long long most = std::max(1LL, (long long)(e->sens_limit.bytes / (slots * kKeptBytes)));
+    const long long batches = (all + most - 1) / most;
+    batch = (all + batches - 1) / batches;
+    if (!use_tangents(batch, K, e->sms, batches > 1 ? 2 * kDualWaves : kDualWaves)) break;
+    const size_t need = slots * batch * kKeptBytes;
+    split = e->sens_kept.reserve(need) == SPI_OK;
+    if (!split) e->sens_limit.refused(need);
+  }
   if (!split) batch = all;
   // The results are the caller's and the directions' own rollouts share nothing, so calls on several streams
   // (spi_set_stream) may overlap; the kept substeps are the engine's, and a call on another stream waits for them.

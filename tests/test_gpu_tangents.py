@@ -82,3 +82,38 @@ def test_each_direction_agrees_with_its_dual_rollout(built, start, kw):
         assert torch.equal(x[n], rx[0])
         err, size = (torch.linalg.norm(a.reshape(-1, 13), dim=0) for a in (J[n] - ref[0], ref[0]))
         assert (err <= 1e-4 * size).all(), (n, err, size)
+
+
+def test_little_memory_takes_smaller_batches(built):
+    """70,000 windows keep 4.2 GB in one batch. With 3 GB left, every call succeeds and gives the bits that it gives
+    with all of it (a window does not depend on its batch); with 0.1 GB left they are the dual rollouts'."""
+    from spi_gb300.data import standing_state
+    from spi_gb300.engine import Engine
+    from spi_gb300.sensitivity import sensitivities
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    init = torch.from_numpy(standing_state(70000)).cuda()
+    actions = 1.2 * torch.rand((70000, 20, 12), device="cuda", generator=gen) - 0.6
+    th = torch.from_numpy(random_theta(np.random.default_rng(2), 1).astype(np.float32))
+
+    def run(left):
+        e = Engine()
+        e.load_windows(init, actions, init)
+        hog = None
+        torch.cuda.empty_cache()
+        spare = torch.empty((2, 70000, 37, 13), device="cuda")     # the calls' results come from torch's cache
+        del spare
+        if left:
+            hog = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+        outs = [sensitivities(e, th, range(13)) for _ in range(2)]
+        torch.cuda.synchronize()
+        del hog
+        e.close()
+        assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+        return outs[0]
+    J, x = run(None)
+    J2, x2 = run(3 << 30)
+    assert torch.equal(J, J2) and torch.equal(x, x2)
+    del J2, x2
+    J3, x3 = run(100 << 20)
+    assert torch.equal(x, x3)
+    assert (torch.linalg.norm((J - J3).reshape(-1, 13), dim=0) <= 1e-4 * torch.linalg.norm(J3.reshape(-1, 13), dim=0)).all()
