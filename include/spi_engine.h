@@ -209,8 +209,8 @@ int spi_cem_read(spi_engine* e, double* mu, double* cov, float* best_theta, floa
  * spi_sensitivity: J[n][w][i][k] = d s_H[i] / d theta[param_ids[k]] of window w (the loaded
  * windows) for theta sample n (device [N][13]); J device [N][W][37][K]; xH device
  * [N][W][37] final states or NULL. K <= 13. Three directions or more of many pairs keep the first
- * direction's substeps in engine memory (4 GB at most; without it, and in a stream capture, every
- * direction runs its own rollout). Asynchronous on the engine stream.
+ * direction's substeps in engine memory (4 GB at most, less where the device has less; without it, and in
+ * a stream capture, every direction runs its own rollout). Asynchronous on the engine stream.
  * spi_fisher: F[n] = sum_w J_w^T diag(state_weight) J_w (device [N][K][K], FP32
  * accumulation), logdet[n] = log det(F[n] + eps I) and trace[n] = trace(F[n]) in FP64
  * (device [N] each, may be NULL). */

@@ -107,6 +107,7 @@ def test_little_memory_takes_smaller_batches(built):
         outs = [sensitivities(e, th, range(13)) for _ in range(2)]
         torch.cuda.synchronize()
         del hog
+        torch.cuda.empty_cache()                                   # back to the device, for what allocates outside torch
         e.close()
         assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
         return outs[0]
