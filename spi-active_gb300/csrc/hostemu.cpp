@@ -647,8 +647,8 @@ int spi_hostemu_count_ops_tangent(const spi_robot* robot, const double* state, c
   for (int leg = 0; leg < 4; ++leg) {
     Cf dr[3];
     SV<Cf> dfb;
-    tng::leg_residual_tan(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, qdd[leg], t[leg], t[leg].zf, {true, false}, dB, dL[leg], dP, dr,
-                          dfb);
+    tng::leg_residual_tan(M, leg, B0, L[leg], lp[leg], tgt + 3 * leg, qdd[leg], t[leg], t[leg].zf, {true, false}, dB,
+                          dL[leg], dP, dr, dfb);
     adj::add_sv(x, dfb);
     adj::add_sv(x, adj::leg_solve_down(W[leg], dr, z[leg]));
   }

@@ -3,9 +3,10 @@
 // A substep's accelerations a = (a0, qdd) solve r(x, theta, a) = 0 (adjoint.cuh), so a direction
 // (dx, dtheta) moves them by da = -M'^-1 dr with dr = (dr/dx) dx + (dr/dtheta) dtheta at fixed a. Given the
 // substep's factorisation, a direction costs the tangent of the recursive Newton-Euler residual and
-// two triangular solves: 8,564 operations a substep with the residual itself (5,152 where directions share that)
-// against 15,969 for carrying the direction through the condensation and the Cholesky factorisation. Each function below is the derivative of the function of the same
-// name in adjoint.cuh / dynamics.cuh; for a motion o = X m across a joint, do = X dm + (o x S) dq.
+// two triangular solves: 8,564 operations a substep with the residual itself (5,152 where directions
+// share that) against 15,969 for carrying the direction through the condensation and the Cholesky
+// factorisation. Each function below is the derivative of the function of the same name in
+// adjoint.cuh / dynamics.cuh; for a motion o = X m across a joint, do = X dm + (o x S) dq.
 //
 // The contact's branches (normal force on or off, stick or slip) are given, not decided here: the pass
 // that produced the trajectory hands them over with the foot height, so that the tangent is
